@@ -935,10 +935,11 @@ def coulomb_pass_work(name, N, P, U):
           "coul_fwd_y": 16.0 * (N * N * P + N * P * P) * U,
           "coul_z": 32.0 * N * P * P * U + 8.0 * P ** 3,
           "coul_inv_y": 16.0 * (N * P * P + N * N * P) * U,
+          "coul_yzy": 32.0 * N * N * P * U + 8.0 * P ** 3,     # the y, z, y passes of a plane on chip
           "coul_inv_x": 16.0 * (N * N * P + N ** 3) * U}[name]
     lines = {"coul_fwd_x": N * N, "coul_fwd_y": N * P, "coul_z": 2 * P * P, "coul_inv_y": N * P,
-             "coul_inv_x": N * N}[name]
-    extra = {"coul_fwd_x": 6.0 * N ** 3, "coul_z": 2.0 * P ** 3}.get(name, 0.0)
+             "coul_yzy": 2 * N * P + 2 * P * P, "coul_inv_x": N * N}[name]
+    extra = {"coul_fwd_x": 6.0 * N ** 3, "coul_z": 2.0 * P ** 3, "coul_yzy": 2.0 * P ** 3}.get(name, 0.0)
     return by, (lines * fl + extra) * U
 
 
@@ -1011,7 +1012,7 @@ def eval_roofline(w, prof, nprof, dev, P, ms_step):
     stages = {
         # name: (algorithmic bytes, algorithmic flops) per evaluation
         **{k: coulomb_pass_work(k, N, P, U) for k in ("coul_fwd_x", "coul_fwd_y", "coul_z", "coul_inv_y",
-                                                      "coul_inv_x")},
+                                                      "coul_yzy", "coul_inv_x")},
         "twoe_gemm": (16.0 * G * (n + 2 * U), 2.0 * G * (2 * U) ** 2),
         "rp_gemm": (8.0 * G * 2 * U + 16.0 * G * n * n, 2.0 * G * 2 * U * n * (n + 1)),
         "ke_xy": (16.0 * G * n * 2, 2 * 2 * 2.0 * N ** 3 * N * n),

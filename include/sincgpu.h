@@ -104,7 +104,10 @@ int sincgpu_fft_length(sincgpu_ctx* ctx);
  * CTA; results agree to rounding); "orb_blendq" (1, default: an orbital Krylov
  * call with two mean-field slots folds their reduced potentials and density
  * matrices into one blended potential once, and each Jacobian product reads
- * that; 0: each product reads both slots; results agree to rounding). */
+ * that; 0: each product reads both slots; results agree to rounding);
+ * "coul_half" (1, default: FP64 Coulomb solves on half-length transforms where the
+ * grid has such a plan and the kernel is even in each axis; 0: five passes; results
+ * agree to rounding). */
 int sincgpu_set_option(sincgpu_ctx* ctx, const char* name, long long value);
 /* Current value of an option of sincgpu_set_option (SINCGPU_EINVAL for an unknown name). */
 int sincgpu_get_option(sincgpu_ctx* ctx, const char* name, long long* value);

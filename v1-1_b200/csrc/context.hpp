@@ -169,6 +169,12 @@ struct Ctx {
   // is too: khat(P-k) = khat(k)): for P <= 128 on the octant k <= P/2 of each axis,
   // (P/2+1)^3 values; for longer lengths the full P^3 table (khr_len(P) values)
   double* d_khr = nullptr;
+  // half-length form of the Coulomb passes (coulomb_half.cuh): M = hM1 hM2 >= N, or
+  // hM = 0 where it does not apply (no such plan, a kernel that is not even in each
+  // axis); the spectrum at 2M points per axis and the twiddles
+  int hM = 0;
+  double* d_kht = nullptr;
+  double2* d_htw = nullptr;
   float* d_khr32 = nullptr;
   float* d_khT32 = nullptr;
 
@@ -197,6 +203,7 @@ struct Ctx {
   int coul_chunk = 0;   // pairs per pass sequence (0 = automatic)
   int coul_fp32 = 0;    // 1: Coulomb passes in FP32 (precision form), 0: FP64
   int contract_tf32 = 0;  // 1: reducedpot contraction as 3xTF32 on the tensor cores
+  int coul_half = 1;      // 1: FP64 Coulomb solves on half-length transforms where hM > 0, 0: five passes
   int coul_tma = -1;      // TMA-staged persistent z pass: 1 on, 0 off, -1 automatic (off)
   int tc_pipe = 4;        // tcgen05 3xTF32 GEMM with a staging ring and an MMA-issuing warp: 1: 3 stages of
                           // K = 16, 2: 4 x 16, 3: 6 x 8; 4, 5: pre-split operands moved by bulk copies
@@ -294,6 +301,10 @@ int make_khat(Ctx& c);
 int ensure_fp32_tables(Ctx& c);
 // real kernel spectrum transposed to [kx][kz][ky] (FP64, and FP32 with fp32)
 int ensure_khT(Ctx& c, bool fp32);
+
+// tables of the half-length Coulomb form for c.d_tcoul; `even`: the kernel is even in
+// each axis by construction (else it is checked)
+int make_half(Ctx& c, bool even);
 
 // coulomb.cu: R_p = T * (phi1_a conj(phi2_b)) for pairs p=(a_p,b_p).
 // Rpl (device) receives the planar real/imag parts: Rpl[p*G+x] = Re, Rpl[(npair+p)*G+x] = Im.

@@ -1,0 +1,7 @@
+// Explicit instantiations of the half-length Coulomb passes for a group of lengths
+// (split across files so that nvcc compiles them in parallel).
+#include "coulomb_half.cuh"
+namespace sincgpu {
+SINCGPU_HALF_INSTANTIATE(7, 7)
+SINCGPU_HALF_INSTANTIATE(7, 8)
+}  // namespace sincgpu

@@ -25,6 +25,7 @@
 #include <vector>
 #include <cudaTypedefs.h>
 #include "coulomb_kernels.cuh"
+#include "coulomb_half.cuh"
 
 namespace sincgpu {
 
@@ -122,6 +123,36 @@ static bool make_zmap(const Ctx& c, const C* W2, int np, CUtensorMap* map) {
   return r == CUDA_SUCCESS;
 }
 
+// orbitals arriving in groups (host-array entry): the hermitian pair list is b-major
+// (a <= b), so the pairs of orbitals below e are its first e (e + 1) / 2; a chunk
+// never crosses a group's end and the first chunk of each group waits for it
+struct UploadGroups {
+  Ctx& c;
+  const bool on;
+  int g = -1;
+  static int pairs_below(int e) { return e * (e + 1) / 2; }
+  // pairs of the chunk at p0, at most np
+  int next(int p0, int np, int* rc) {
+    *rc = SINCGPU_OK;
+    if (!on) return np;
+    int gg = 0;
+    while (gg < c.up_n - 1 && pairs_below(c.up_end[gg]) <= p0) ++gg;
+    if (gg != g) {
+      if (cudaStreamWaitEvent(c.stream, c.ev_up[gg], 0) != cudaSuccess) {
+        set_error("waiting for an orbital group failed");
+        *rc = SINCGPU_ECUDA;
+      }
+      g = gg;
+    }
+    return std::max(1, std::min(np, pairs_below(c.up_end[gg]) - p0));
+  }
+  // every group has been waited for (the last group ends at the last orbital)
+  int finish() {
+    if (on && g != c.up_n - 1) SG_CUDA(cudaStreamWaitEvent(c.stream, c.ev_up[c.up_n - 1], 0));
+    return SINCGPU_OK;
+  }
+};
+
 template <class C>
 static int coul_run_t(Ctx& c, const double2* src1, const double2* src2, const int* h_pa,
                       const int* h_pb, int npair, double* Rpl, double2* full, bool herm, bool dens) {
@@ -177,36 +208,94 @@ static int coul_run_t(Ctx& c, const double2* src1, const double2* src2, const in
     SG_TRY(timeout_flags(c, &err));
     err += 1;
   }
-  // orbitals arriving in groups (host-array entry): the hermitian pair list is
-  // b-major (a <= b), so the pairs of orbitals below e are its first e (e + 1) / 2;
-  // a chunk never crosses a group's end and the first chunk of each group waits for it
-  const bool grouped = !dens && herm && c.up_n > 0;
-  auto pairs_below = [](int e) { return e * (e + 1) / 2; };
-  int g = -1;
+  UploadGroups up{c, !dens && herm && c.up_n > 0};
   for (int p0 = 0; p0 < npair;) {
-    int np = std::min(chunk, npair - p0);
-    if (grouped) {
-      int gg = 0;
-      while (gg < c.up_n - 1 && pairs_below(c.up_end[gg]) <= p0) ++gg;
-      if (gg != g) {
-        SG_CUDA(cudaStreamWaitEvent(c.stream, c.ev_up[gg], 0));
-        g = gg;
-      }
-      np = std::max(1, std::min(np, pairs_below(c.up_end[gg]) - p0));
-    }
+    int rc;
+    const int np = up.next(p0, std::min(chunk, npair - p0), &rc);
+    SG_TRY(rc);
     ca.pair0 = p0;
     ca.pa = d_pa ? d_pa + p0 : nullptr;
     ca.pb = d_pb ? d_pb + p0 : nullptr;
     SG_TRY(coul_dispatch(c, ca, np, dens, src1, src2, Rpl, full, herm, use_tma ? &zmap : nullptr, err));
     p0 += np;
   }
-  // every group has been waited for (the last group ends at the last orbital)
-  if (grouped && g != c.up_n - 1) SG_CUDA(cudaStreamWaitEvent(c.stream, c.ev_up[c.up_n - 1], 0));
-  return SINCGPU_OK;
+  return up.finish();
+}
+
+// The half-length form serves FP64 solves with the options of the other forms off.
+static bool use_half(const Ctx& c) {
+  return c.coul_half && c.hM > 0 && !c.coul_fp32 && c.coul_fused == 0 && c.coul_tma <= 0 && !c.coul_z2;
+}
+
+static long long half_places(const Ctx& c) {
+  int m1 = 0, m2 = 0;
+  half_length_for(c.N, &m1, &m2);
+  return half_slots(c.N, m1, m2);
+}
+// bytes of W and V per pair
+static long long half_pair_bytes(const Ctx& c) {
+  return 2LL * (long long)sizeof(double2) * 2 * c.hM * half_places(c);
+}
+
+static HalfArgs half_args(const Ctx& c, void* scratch, int chunk, int npair, bool herm) {
+  HalfArgs ha{};
+  ha.N = c.N;
+  ha.nspf = c.nspf;
+  ha.herm = herm ? 1 : 0;
+  ha.G = c.G;
+  ha.NS = half_places(c);
+  ha.tw = c.d_htw;
+  ha.kht = c.d_kht;
+  ha.W = (double2*)scratch;
+  ha.V = ha.W + (long long)chunk * 2 * c.hM * ha.NS;
+  ha.npair_total = npair;
+  return ha;
+}
+
+static int half_dispatch(Ctx& c, const HalfArgs& ha, int np, bool dens, const double2* s1, const double2* s2,
+                         double* Rpl, double2* full) {
+  switch (c.hM) {
+#define SINCGPU_CASE(M, A, B, NMIN) \
+  case M:                           \
+    return half_launch<A, B>(c, ha, np, dens, s1, s2, Rpl, full);
+    SINCGPU_HALF_LENGTHS(SINCGPU_CASE)
+#undef SINCGPU_CASE
+    default:
+      set_error("no Coulomb kernels for half-length %d", c.hM);
+      return SINCGPU_ERANGE;
+  }
+}
+
+static int half_run(Ctx& c, const double2* src1, const double2* src2, const int* h_pa, const int* h_pb, int npair,
+                    double* Rpl, double2* full, bool herm, bool dens) {
+  const long long per_pair = half_pair_bytes(c);
+  int chunk = c.coul_chunk;
+  if (chunk <= 0) chunk = (int)std::min(65535LL, std::max(1LL, kCoulChunkBudget / per_pair));
+  chunk = std::min(chunk, npair);
+  SG_TRY(c.ws_fft.ensure((size_t)per_pair * chunk));
+  const int *d_pa = nullptr, *d_pb = nullptr;
+  if (!dens) {
+    SG_TRY(cached_ints(c, IC_PA, h_pa, npair, &d_pa));
+    SG_TRY(cached_ints(c, IC_PB, h_pb, npair, &d_pb));
+  }
+  HalfArgs ha = half_args(c, c.ws_fft.ptr, chunk, npair, herm);
+  UploadGroups up{c, !dens && herm && c.up_n > 0};
+  for (int p0 = 0; p0 < npair;) {
+    int rc;
+    const int np = up.next(p0, std::min(chunk, npair - p0), &rc);
+    SG_TRY(rc);
+    ha.pair0 = p0;
+    ha.pa = d_pa ? d_pa + p0 : nullptr;
+    ha.pb = d_pb ? d_pb + p0 : nullptr;
+    SG_TRY(half_dispatch(c, ha, np, dens, src1, src2, Rpl, full));
+    p0 += np;
+  }
+  return up.finish();
 }
 
 static int coul_run(Ctx& c, const double2* src1, const double2* src2, const int* h_pa,
                     const int* h_pb, int npair, double* Rpl, double2* full, bool herm, bool dens) {
+  if (use_half(c)) return half_run(c, src1, src2, h_pa, h_pb, npair, Rpl, full, herm, dens);
   if (c.coul_fp32) {
     SG_TRY(ensure_fp32_tables(c));
     return coul_run_t<float2>(c, src1, src2, h_pa, h_pb, npair, Rpl, full, herm, dens);
@@ -233,6 +322,16 @@ static int coulomb_dens_scratch_t(Ctx& c, const double2* dens, int m, double2* r
   SG_CHECK(per_dens <= scratch_bytes, SINCGPU_ERANGE,
            "one density on a %d^3 grid (FFT length %d) needs %zu bytes of scratch; the fixed "
            "scratch holds %zu bytes", N, P, per_dens, scratch_bytes);
+  if (use_half(c)) {  // less than the five passes need, or (N <= 21) far less than the scratch
+    const size_t per = (size_t)half_pair_bytes(c);
+    const int chunk = (int)std::min<size_t>({scratch_bytes / per, (size_t)m, 65535});
+    HalfArgs ha = half_args(c, scratch, chunk, m, false);
+    for (int p0 = 0; p0 < m; p0 += chunk) {
+      ha.pair0 = p0;
+      SG_TRY(half_dispatch(c, ha, std::min(chunk, m - p0), true, dens, nullptr, nullptr, red));
+    }
+    return SINCGPU_OK;
+  }
   const int chunk = (int)std::min<size_t>(scratch_bytes / per_dens, (size_t)m);
   CoulArgs<C> ca{};
   ca.N = N;

@@ -12,6 +12,7 @@
 #include <mutex>
 #include <set>
 #include "context.hpp"
+#include "coul_half.h"
 #include "fft_lengths.h"
 
 namespace sincgpu {
@@ -53,10 +54,8 @@ static bool smooth7(int p) {
 
 int fft_length_for(int min_len, int* p1, int* p2);  // coulomb.cu
 
-int choose_plan(Ctx& c) {
-  int P = fft_length_for(2 * c.N - 1, nullptr, nullptr);
-  SG_CHECK(P > 0 && P <= kMaxFftLen && smooth7(P), SINCGPU_ERANGE,
-           "no supported padded FFT length >= %d (N=%d)", 2 * c.N - 1, c.N);
+// stages of a 7-smooth length (4, 2, 3, 5, 7)
+static int plan_for(int P, FftPlan* plan) {
   FftPlan pl{};
   pl.P = P;
   int p = P, k = 0;
@@ -68,22 +67,33 @@ int choose_plan(Ctx& c) {
     }
   }
   pl.nrad = k;
-  c.plan = pl;
-  c.P = P;
-  // column tile: largest divisor of P in [8,32] whose double buffer fits 100 KB
-  int tx = 0;
+  *plan = pl;
+  return SINCGPU_OK;
+}
+// column tile: largest divisor of P in [8,32] whose double buffer fits 100 KB
+static int column_tile(int P) {
   for (int t = 32; t >= 8; --t)
-    if (P % t == 0 && 2LL * P * t * 16 <= 100 * 1024) {
-      tx = t;
-      break;
-    }
-  if (tx == 0) tx = 16;
-  c.tx = tx;
+    if (P % t == 0 && 2LL * P * t * 16 <= 100 * 1024) return t;
+  return 16;
+}
+// exp(-2 pi i m / P), m < P
+static std::vector<double2> host_roots(int P) {
   std::vector<double2> roots(P);
   for (int m = 0; m < P; ++m) {
     long double ang = -2.0L * 3.14159265358979323846264338327950288L * (long double)m / (long double)P;
     roots[m] = make_double2((double)cosl(ang), (double)sinl(ang));
   }
+  return roots;
+}
+
+int choose_plan(Ctx& c) {
+  int P = fft_length_for(2 * c.N - 1, nullptr, nullptr);
+  SG_CHECK(P > 0 && P <= kMaxFftLen && smooth7(P), SINCGPU_ERANGE,
+           "no supported padded FFT length >= %d (N=%d)", 2 * c.N - 1, c.N);
+  SG_TRY(plan_for(P, &c.plan));
+  c.P = P;
+  c.tx = column_tile(P);
+  const std::vector<double2> roots = host_roots(P);
   SG_TRY(dupload(c, (void**)&c.d_roots, roots.data(), sizeof(double2) * P));
   return SINCGPU_OK;
 }
@@ -496,6 +506,127 @@ __global__ void narrow_real_kernel(float* __restrict__ out, const double* __rest
     out[i] = (float)in[i];
 }
 
+// spec = DFT of the kernel c.d_tcoul on plan.P^3 points / plan.P^3
+static int kernel_spectrum(Ctx& c, const FftPlan& plan, int tx, const double2* roots, double2* spec) {
+  const int P = plan.P;
+  const long long P3 = (long long)P * P * P;
+  embed_kernel<<<ceil_div(P3, 256), 256, 0, c.stream>>>(spec, c.d_tcoul, c.N, P);
+  SG_LAUNCHED();
+  size_t sm0 = sizeof(double2) * (P + 2 * 8 * (P + 1));
+  size_t sm1 = sizeof(double2) * (P + 2 * P * tx);
+  size_t smax = std::max(sm0, sm1);
+  // the attribute is process-wide: always the same (largest) value, so contexts
+  // created concurrently on several threads never lower it under each other
+  constexpr int kSmemOptIn = 227 * 1024;
+  SG_CHECK(smax <= (size_t)kSmemOptIn, SINCGPU_ERANGE, "kernel-spectrum FFT needs %zu bytes of shared memory", smax);
+  SG_CUDA(cudaFuncSetAttribute(fft_full_axis_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn));
+  fft_full_axis_kernel<<<ceil_div((long long)P * P, 8), 128, sm0, c.stream>>>(spec, plan, roots, 0, tx, 1.0);
+  SG_LAUNCHED();
+  dim3 g1(ceil_div(P, tx), P);
+  fft_full_axis_kernel<<<g1, 128, sm1, c.stream>>>(spec, plan, roots, 1, tx, 1.0);
+  SG_LAUNCHED();
+  const double inv = 1.0 / ((double)P * (double)P * (double)P);
+  fft_full_axis_kernel<<<g1, 128, sm1, c.stream>>>(spec, plan, roots, 2, tx, inv);
+  SG_LAUNCHED();
+  return SINCGPU_OK;
+}
+
+// the kernel spectrum in the order of the half-length z transforms (half_spec_plane):
+// kht[(((fx 2 + py) 2 + pz) groups + gi) m2 + k2][i] = Re spec(fx, fy, fz) / scale for
+// thread i = sc LG + lc of column group gi, i.e. the column at position q = gi LG + lc
+// of parity py and its frequency (sc, k2) of parity pz; unused places are zero
+__global__ void half_table_kernel(double* __restrict__ kht, const double2* __restrict__ spec, int m1, int m2,
+                                  long long len) {
+  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (idx >= len) return;
+  const int M = m1 * m2, L = 2 * M, LG = half_lines(m1, m2), groups = half_col_groups(m1, m2);
+  const int i = (int)(idx % 64), k2 = (int)((idx / 64) % m2), gi = (int)((idx / (64LL * m2)) % groups);
+  const int pp = (int)((idx / (64LL * m2 * groups)) % 4), fx = (int)(idx / (256LL * m2 * groups));
+  const int py = pp >> 1, pz = pp & 1;
+  const int sc = i / LG, q = gi * LG + i % LG;
+  double v = 0.0;
+  if (sc < m1 && q < M) {
+    const int fy = half_freq2(m1, m2, q / m2, q % m2, py), fz = half_freq2(m1, m2, sc, k2, pz);
+    v = spec[((long long)fz * L + fy) * L + fx].x;
+  }
+  kht[idx] = v;
+}
+
+// out[0] = max |T(d) - T with one axis mirrored|, out[1] = max |T| (bit patterns of
+// non-negative doubles order like integers; a NaN exceeds every number)
+__global__ void even_kernel(const double* __restrict__ T, int W, unsigned long long* __restrict__ out) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= (long long)W * W * W) return;
+  const int a = (int)(i % W), b = (int)((i / W) % W), d = (int)(i / ((long long)W * W));
+  const double t = T[i];
+  const double m[3] = {T[(W - 1 - a) + (long long)W * (b + (long long)W * d)],
+                       T[a + (long long)W * ((W - 1 - b) + (long long)W * d)],
+                       T[a + (long long)W * (b + (long long)W * (W - 1 - d))]};
+  for (int k = 0; k < 3; ++k) atomicMax(out, (unsigned long long)__double_as_longlong(fabs(t - m[k])));
+  atomicMax(out + 1, (unsigned long long)__double_as_longlong(fabs(t)));
+}
+
+int make_half(Ctx& c, bool even) {
+  dfree(c, c.d_kht);
+  dfree(c, c.d_htw);
+  c.d_kht = nullptr;
+  c.d_htw = nullptr;
+  c.hM = 0;
+  int m1 = 0, m2 = 0;
+  const int M = half_length_for(c.N, &m1, &m2);
+  if (M < 0) return SINCGPU_OK;
+  if (!even) {
+    // the spectrum is read on one octant, so a caller's kernel has to be even in each
+    // axis to rounding; another one keeps the five passes
+    const long long W = 2LL * c.N - 1;
+    unsigned long long* d = nullptr;
+    unsigned long long h[2];
+    SG_TRY(dalloc(c, &d, sizeof(h)));
+    SG_CUDA(cudaMemsetAsync(d, 0, sizeof(h), c.stream));
+    even_kernel<<<ceil_div(W * W * W, 256), 256, 0, c.stream>>>(c.d_tcoul, (int)W, d);
+    SG_LAUNCHED();
+    SG_CUDA(cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, c.stream));
+    SG_CUDA(cudaStreamSynchronize(c.stream));
+    dfree(c, d);
+    double v[2];
+    std::memcpy(v, h, sizeof(v));
+    if (!(v[0] <= 1e-14 * v[1])) return SINCGPU_OK;
+  }
+  const int L = 2 * M;
+  const std::vector<double2> roots = host_roots(L);
+  // [parity p][k < m1][s, rows of ts] = w_L^(s (2 k + p)), the even parity alone for odd M
+  const int ts = m2 | 1, np = M % 2 ? 1 : 2;
+  std::vector<double2> tw((size_t)np * m1 * ts, make_double2(0.0, 0.0));
+  for (int p = 0; p < np; ++p)
+    for (int k = 0; k < m1; ++k)
+      for (int s = 0; s < m2; ++s) tw[(size_t)(p * m1 + k) * ts + s] = roots[s * (2 * k + p)];
+  SG_TRY(dupload(c, (void**)&c.d_htw, tw.data(), sizeof(double2) * tw.size()));
+  double2* spec = c.d_khat;
+  if (L != c.P) {
+    FftPlan plan;
+    SG_TRY(plan_for(L, &plan));
+    spec = nullptr;
+    SG_TRY(dalloc(c, &spec, sizeof(double2) * (long long)L * L * L));
+    double2* d_roots = nullptr;
+    int rc = dupload(c, (void**)&d_roots, roots.data(), sizeof(double2) * L);
+    if (rc == SINCGPU_OK) rc = kernel_spectrum(c, plan, column_tile(L), d_roots, spec);
+    dfree(c, d_roots);
+    if (rc != SINCGPU_OK) {
+      dfree(c, spec);
+      return rc;
+    }
+  }
+  const long long len = (long long)(M + 1) * half_spec_plane(m1, m2);
+  const int rc = dalloc(c, &c.d_kht, sizeof(double) * len);
+  if (rc == SINCGPU_OK) half_table_kernel<<<ceil_div(len, 256), 256, 0, c.stream>>>(c.d_kht, spec, m1, m2, len);
+  if (spec != c.d_khat) dfree(c, spec);
+  SG_TRY(rc);
+  SG_LAUNCHED();
+  SG_CUDA(cudaStreamSynchronize(c.stream));
+  c.hM = M;
+  return SINCGPU_OK;
+}
+
 int make_khat(Ctx& c) {
   const int P = c.P;
   const long long P3 = (long long)P * P * P;
@@ -514,25 +645,7 @@ int make_khat(Ctx& c) {
   c.d_khT = nullptr;
   c.d_khT32 = nullptr;
   SG_TRY(dalloc(c, &c.d_khat, sizeof(double2) * P3));
-  embed_kernel<<<ceil_div(P3, 256), 256, 0, c.stream>>>(c.d_khat, c.d_tcoul, c.N, P);
-  SG_LAUNCHED();
-  size_t sm0 = sizeof(double2) * (P + 2 * 8 * (P + 1));
-  size_t sm1 = sizeof(double2) * (P + 2 * P * c.tx);
-  size_t smax = std::max(sm0, sm1);
-  // the attribute is process-wide: always the same (largest) value, so contexts
-  // created concurrently on several threads never lower it under each other
-  constexpr int kSmemOptIn = 227 * 1024;
-  SG_CHECK(smax <= (size_t)kSmemOptIn, SINCGPU_ERANGE, "kernel-spectrum FFT needs %zu bytes of shared memory", smax);
-  SG_CUDA(cudaFuncSetAttribute(fft_full_axis_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn));
-  fft_full_axis_kernel<<<ceil_div((long long)P * P, 8), 128, sm0, c.stream>>>(c.d_khat, c.plan, c.d_roots, 0,
-                                                                              c.tx, 1.0);
-  SG_LAUNCHED();
-  dim3 g1(ceil_div(P, c.tx), P);
-  fft_full_axis_kernel<<<g1, 128, sm1, c.stream>>>(c.d_khat, c.plan, c.d_roots, 1, c.tx, 1.0);
-  SG_LAUNCHED();
-  const double inv = 1.0 / ((double)P * (double)P * (double)P);
-  fft_full_axis_kernel<<<g1, 128, sm1, c.stream>>>(c.d_khat, c.plan, c.d_roots, 2, c.tx, inv);
-  SG_LAUNCHED();
+  SG_TRY(kernel_spectrum(c, c.plan, c.tx, c.d_roots, c.d_khat));
   const long long nkr = khr_len(P);
   SG_TRY(dalloc(c, &c.d_khr, sizeof(double) * nkr));
   khat_real_kernel<<<ceil_div(nkr, 256), 256, 0, c.stream>>>(c.d_khr, c.d_khat, P);
@@ -612,7 +725,7 @@ int build_tables(Ctx& c, int toothnbig, int toothnsmall, int flags) {
     SG_CUDA(cudaMemsetAsync(c.d_tcoul, 0, sizeof(double) * W * W * W, c.stream));
   }
   SG_TRY(make_khat(c));
-  return SINCGPU_OK;
+  return make_half(c, true);
 }
 
 // threed_two(-N:N-1)^3 (complex, real valued) and pot supplied by the caller,
@@ -656,7 +769,7 @@ int build_tables_from_arrays(Ctx& c, const double2* threed_two_host, const doubl
   e = cudaStreamSynchronize(c.stream);
   SG_CHECK(e == cudaSuccess, SINCGPU_ECUDA, "zdip: %s", cudaGetErrorString(e));
   SG_TRY(make_khat(c));
-  return SINCGPU_OK;
+  return make_half(c, false);
 }
 
 }  // namespace sincgpu
