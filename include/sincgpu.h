@@ -99,9 +99,9 @@ int sincgpu_fft_length(sincgpu_ctx* ctx);
  * a copy stream, and the Coulomb pair loop starts on the pairs of the first
  * group while the others are in flight; 1: one copy before the evaluation;
  * bitwise the same); "kry_cluster" (1, default: the A-vector Krylov's
- * Gram-Schmidt step on vectors longer than 4096 reals runs on a cluster of 8
- * CTAs with the dot products summed through distributed shared memory; 0: one
- * CTA; results agree to rounding); "orb_blendq" (1, default: an orbital Krylov
+ * Gram-Schmidt step and update run on a cluster of 8 CTAs, its coefficients from one
+ * pass of dot products summed through distributed shared memory, for vectors of up to
+ * 112640 reals; 0: one CTA, one projection after another; results agree to rounding); "orb_blendq" (1, default: an orbital Krylov
  * call with two mean-field slots folds their reduced potentials and density
  * matrices into one blended potential once, and each Jacobian product reads
  * that; 0: each product reads both slots; results agree to rounding);

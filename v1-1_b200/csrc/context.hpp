@@ -217,7 +217,7 @@ struct Ctx {
   int twoe_symdiag = 0;   // 1: multi-tile twoematel computes its diagonal tiles' lower blocks only
   int twoe_tile = 0;      // twoematel tile edge 16R: 0 = least padding, 2..9 = that R
   int orth_fused = 1;     // 1: an orbital Arnoldi step's orthogonalisation in one cooperative launch
-  int kry_cluster = 1;    // 1: A-vector Gram-Schmidt beyond 4096 reals on a cluster of CTAs (0: one CTA)
+  int kry_cluster = 1;    // 1: A-vector Gram-Schmidt and update on a cluster of CTAs (0: one CTA)
   int orb_blendq = 1;     // 1: the orbital Jacobian reads one blended reduced potential (0: both slots')
   int rhs_overlap = 1;    // 1: the fused orbital-RHS entry runs its CI part and the mix + kinetic
                           //    contraction on `side`, beside the Coulomb passes and twoematel
@@ -383,6 +383,9 @@ int ci_tally(Ctx& c, const double2* a1, const double2* a2, double2* tally);
 int ci_onebody(Ctx& c, const double2* phi, double2* mats);
 int ci_assemble(Ctx& c, const double2* twoematel, const double2* mats);
 int ci_sigma(Ctx& c, const double2* in, double2* out, double constant, double ez, double nucdipz);
+// the same times tf, and nothing where the device flag *skip is set
+int ci_sigma(Ctx& c, const double2* in, double2* out, double constant, double ez, double nucdipz, double2 tf,
+             const int* skip);
 int ci_dipole_z(Ctx& c, const double2* a, double2* tmp, double nucdipz, double2* dip, double* normsq);
 
 // krylov.cu: w = exp(t * timefac * H) v on the real-ified A-vector

@@ -92,162 +92,182 @@ __global__ void __launch_bounds__(kKryThreads) kry_mgs_kernel(double* __restrict
   for (long long k = threadIdx.x; k < n; k += blockDim.x) p[k] *= inv;
 }
 
-// kry_mgs_kernel with p held in registers (the same elements per thread,
-// k = threadIdx.x + e blockDim.x, and the same sums in the same order: the same
-// bits) and v_{i+1} loaded while v_i's projection is being reduced, so that no
-// global access sits inside the sequential loop.  n <= E * kKryThreads.
-template <int E>
-__global__ void __launch_bounds__(kKryThreads) kry_mgs_reg_kernel(double* __restrict__ V, long long n, int j,
-                                                                  double* __restrict__ Hm, int mh,
-                                                                  double break_tol, KryState* st) {
-  __shared__ double red[33];
-  if (st->mbrk) return;
-  double* p = V + (long long)(j + 1) * n;
-  double x[E], a[E], an[E];
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const long long k = threadIdx.x + (long long)e * blockDim.x;
-    x[e] = k < n ? p[k] : 0.0;
-    a[e] = k < n ? V[k] : 0.0;
-    an[e] = 0.0;
-  }
-  for (int i = 0; i <= j; ++i) {
-    if (i < j) {
-      const double* vn = V + (long long)(i + 1) * n;
-#pragma unroll
-      for (int e = 0; e < E; ++e) {
-        const long long k = threadIdx.x + (long long)e * blockDim.x;
-        an[e] = k < n ? vn[k] : 0.0;
-      }
-    }
-    double s = 0.0;
-#pragma unroll
-    for (int e = 0; e < E; ++e)
-      if (threadIdx.x + (long long)e * blockDim.x < n) s += a[e] * x[e];
-    const double hij = block_sum(s, red);
-#pragma unroll
-    for (int e = 0; e < E; ++e)
-      if (threadIdx.x + (long long)e * blockDim.x < n) x[e] -= hij * a[e];
-    if (threadIdx.x == 0) Hm[(long long)j * mh + i] = hij;
-    __syncthreads();
-#pragma unroll
-    for (int e = 0; e < E; ++e) a[e] = an[e];
-  }
-  double s = 0.0;
-#pragma unroll
-  for (int e = 0; e < E; ++e)
-    if (threadIdx.x + (long long)e * blockDim.x < n) s += x[e] * x[e];
-  const double h = sqrt(block_sum(s, red));
-  const bool brk = h <= break_tol;
-  if (threadIdx.x == 0) {
-    if (brk) st->mbrk = j + 1;
-    else Hm[(long long)j * mh + j + 1] = h;
-  }
-  const double inv = 1.0 / h;
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const long long k = threadIdx.x + (long long)e * blockDim.x;
-    if (k < n) p[k] = brk ? x[e] : x[e] * inv;
-  }
-}
+// One Arnoldi step's orthogonalisation on a thread-block cluster: the modified
+// Gram-Schmidt coefficients from one pass of dots.  With r_i = <v_i, p> and
+// L_ik = <v_i, v_k> (k < i; rounding level), the sequential projections' h solve
+// (I + L) h = r, so h = r - L r up to L^2, which is far below rounding (L is some
+// eps / break_tol at most): the same coefficients and the same loss of orthogonality
+// as kry_mgs_kernel to rounding, without its j + 1 dependent sums.  Row j of L is
+// formed in the same pass over V (v_j is a row already) and kept for later steps.
+//
+// CTA q of the cluster owns the slice [q S, q S + S) of the vectors, S = ceil(n /
+// kGsCluster) rounded up to even; p and v_j of the slice sit in shared memory.  Warp w
+// sums the dots of rows w, w + 32, ...; the CTAs' partials are added in rank order
+// through distributed shared memory, so every CTA gets the same value.
+// What bounds it: the latency of four dependent stages (loads of p, dots, update, norm)
+// and two cluster barriers, 12 to 14 us a step with cold caches, against j + 2
+// dependent sums in one CTA (784 determinants, 30 vectors: 21.9 us a step) or over the
+// cluster (3136 determinants: 32.6 us).  One A-vector step of 30 vectors at 3136
+// determinants: 1627 -> 901 us, with the sigma product's scaling folded in and the
+// cluster form of the update (94 -> 20 us).
+constexpr int kGsCluster = 8;
+constexpr long long kGsSlice = 14080;  // values of a slice: p and v_j in 220 KB
 
-// kry_mgs_reg_kernel over a thread-block cluster of kMgsCluster CTAs, for vectors
-// longer than one CTA holds in registers (n > 4 kKryThreads): CTA r of the cluster
-// keeps the slice [r S, r S + S) of p in registers (S = ceil(n / kMgsCluster),
-// E elements per thread), each projection's dot is summed per CTA (block_sum) and
-// then over the cluster's partials in rank order through distributed shared memory
-// (so every CTA gets the same value, and the sums have a fixed shape), one cluster
-// barrier per sum (the partials alternate between two slots).  The modified
-// Gram-Schmidt order of expokit.f90:2327-2346 is kept; only the shape of each sum
-// differs from the single-CTA kernels.  A single CTA took 0.37 ms per call at
-// 28800 reals (14400 determinants): its loads of V sat behind one SM's bandwidth.
-constexpr int kMgsCluster = 8;
-
-template <int E>
-__global__ void __launch_bounds__(kKryThreads) kry_mgs_cluster_kernel(double* __restrict__ V, long long n, int j,
-                                                                      double* __restrict__ Hm, int mh,
-                                                                      double break_tol, KryState* st) {
+__global__ void __launch_bounds__(kKryThreads) kry_gs_kernel(double* __restrict__ V, long long n, int S, int j,
+                                                             double* __restrict__ Hm, int mh,
+                                                             double* __restrict__ Lm, double break_tol, KryState* st) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
+  extern __shared__ double gsm[];  // p slice, v_j slice
   __shared__ double red[33];
-  __shared__ double cpart[2];
+  __shared__ double part[2][128];  // this CTA's partial dots <v_i, p>, <v_i, v_j>
+  __shared__ double npart, r[128], lrow[128], h[128];
   if (st->mbrk) return;  // the same value in every CTA of the cluster
-  const long long S = (n + kMgsCluster - 1) / kMgsCluster;
-  const long long lo = (long long)cl.block_rank() * S, hi = min(n, lo + S);
-  double* p = V + (long long)(j + 1) * n;
-  int nsum = 0;
-  // sum over the cluster: this CTA's block sum, then the kMgsCluster partials in rank order
-  auto cluster_sum = [&](double v) {
-    const double b = block_sum(v, red);
-    const int slot = nsum++ & 1;
-    if (threadIdx.x == 0) cpart[slot] = b;
-    cl.sync();
-    double t = 0.0;
-#pragma unroll
-    for (int q = 0; q < kMgsCluster; ++q) t += *cl.map_shared_rank(&cpart[slot], q);
-    return t;
-  };
-  double x[E], a[E], an[E];
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const long long k = lo + threadIdx.x + (long long)e * blockDim.x;
-    x[e] = k < hi ? p[k] : 0.0;
-    a[e] = k < hi ? V[k] : 0.0;
-    an[e] = 0.0;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const long long lo = (long long)cl.block_rank() * S;
+  const int len = (int)max(0LL, min((long long)S, n - lo));
+  double* ps = gsm;
+  double* vs = gsm + S;
+  const double* vj = V + (long long)j * n + lo;
+  double* pg = V + (long long)(j + 1) * n + lo;
+  for (int k = tid; k < len; k += kKryThreads) {
+    ps[k] = pg[k];
+    vs[k] = vj[k];
   }
-  for (int i = 0; i <= j; ++i) {
-    if (i < j) {
-      const double* vn = V + (long long)(i + 1) * n;
-#pragma unroll
-      for (int e = 0; e < E; ++e) {
-        const long long k = lo + threadIdx.x + (long long)e * blockDim.x;
-        an[e] = k < hi ? vn[k] : 0.0;
-      }
+  __syncthreads();
+  for (int i = warp; i <= j; i += kKryThreads / 32) {
+    const double* vi = V + (long long)i * n + lo;
+    double a = 0.0, b = 0.0;
+    int k = lane;
+    for (; k + 96 < len; k += 128) {
+      const double v0 = vi[k], v1 = vi[k + 32], v2 = vi[k + 64], v3 = vi[k + 96];
+      a = fma(v3, ps[k + 96], fma(v2, ps[k + 64], fma(v1, ps[k + 32], fma(v0, ps[k], a))));
+      b = fma(v3, vs[k + 96], fma(v2, vs[k + 64], fma(v1, vs[k + 32], fma(v0, vs[k], b))));
     }
-    double s = 0.0;
-#pragma unroll
-    for (int e = 0; e < E; ++e) s += a[e] * x[e];  // zero outside the slice
-    const double hij = cluster_sum(s);
-#pragma unroll
-    for (int e = 0; e < E; ++e) x[e] -= hij * a[e];
-    if (cl.block_rank() == 0 && threadIdx.x == 0) Hm[(long long)j * mh + i] = hij;
-#pragma unroll
-    for (int e = 0; e < E; ++e) a[e] = an[e];
+    for (; k < len; k += 32) {
+      const double v = vi[k];
+      a = fma(v, ps[k], a);
+      b = fma(v, vs[k], b);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      a += __shfl_down_sync(0xffffffffu, a, o);
+      b += __shfl_down_sync(0xffffffffu, b, o);
+    }
+    if (lane == 0) {
+      part[0][i] = a;
+      part[1][i] = b;
+    }
   }
+  cl.sync();
+  if (tid <= j) {
+    double a = 0.0, b = 0.0;
+#pragma unroll
+    for (int q = 0; q < kGsCluster; ++q) {
+      const double* o = cl.map_shared_rank(&part[0][0], q);
+      a += o[tid];
+      b += o[128 + tid];
+    }
+    r[tid] = a;
+    // row j of L (its diagonal is not used)
+    if (cl.block_rank() == 0 && tid < j) Lm[(long long)j * mh + tid] = b;
+    lrow[tid] = b;
+  }
+  __syncthreads();
+  // h_i = r_i - sum_{k < i} L_ik r_k, a warp per row, the same in every CTA
+  for (int i = warp; i <= j; i += kKryThreads / 32) {
+    double a = 0.0;
+    for (int k = lane; k < i; k += 32) a = fma(i < j ? Lm[(long long)i * mh + k] : lrow[k], r[k], a);
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+    if (lane == 0) {
+      h[i] = r[i] - a;
+      if (cl.block_rank() == 0) Hm[(long long)j * mh + i] = r[i] - a;
+    }
+  }
+  __syncthreads();
   double s = 0.0;
+  for (int k = tid; k < len; k += kKryThreads) {
+    const double* vk = V + lo + k;
+    double x = ps[k];
+    int i = 0;
+    for (; i + 3 <= j; i += 4) {
+      const double v0 = vk[(long long)i * n], v1 = vk[(long long)(i + 1) * n], v2 = vk[(long long)(i + 2) * n],
+                   v3 = vk[(long long)(i + 3) * n];
+      x = fma(-h[i + 3], v3, fma(-h[i + 2], v2, fma(-h[i + 1], v1, fma(-h[i], v0, x))));
+    }
+    for (; i <= j; ++i) x = fma(-h[i], vk[(long long)i * n], x);
+    ps[k] = x;
+    s = fma(x, x, s);
+  }
+  s = block_sum(s, red);
+  if (tid == 0) npart = s;
+  cl.sync();
+  double t = 0.0;
 #pragma unroll
-  for (int e = 0; e < E; ++e) s += x[e] * x[e];
-  const double h = sqrt(cluster_sum(s));
-  const bool brk = h <= break_tol;
-  if (cl.block_rank() == 0 && threadIdx.x == 0) {
+  for (int q = 0; q < kGsCluster; ++q) t += *cl.map_shared_rank(&npart, q);
+  const double hn = sqrt(t);
+  const bool brk = hn <= break_tol;
+  if (cl.block_rank() == 0 && tid == 0) {
     if (brk) st->mbrk = j + 1;
-    else Hm[(long long)j * mh + j + 1] = h;
+    else Hm[(long long)j * mh + j + 1] = hn;
   }
-  const double inv = 1.0 / h;
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const long long k = lo + threadIdx.x + (long long)e * blockDim.x;
-    if (k < hi) p[k] = brk ? x[e] : x[e] * inv;
-  }
+  const double inv = 1.0 / hn;
+  for (int k = tid; k < len; k += kKryThreads) pg[k] = brk ? ps[k] : ps[k] * inv;
   cl.sync();  // no CTA leaves while another may still read its partials
 }
 
-template <int E>
-static int launch_mgs_cluster(Ctx& c, double* V, long long n, int j, double* Hm, int mh, double break_tol,
-                              KryState* st) {
+// w = beta * V[0:mx]^T exph[0:mx]; beta <- |w|, over the same cluster and slices
+__global__ void __launch_bounds__(kKryThreads) kry_update_cluster_kernel(const double* __restrict__ V, long long n,
+                                                                         int S, int mx,
+                                                                         const double* __restrict__ exph,
+                                                                         double* __restrict__ w, KryState* st) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ double red[33], ex[128];
+  __shared__ double npart;
+  const int tid = threadIdx.x;
+  const double beta = st->beta;
+  const long long lo = (long long)cl.block_rank() * S;
+  const int len = (int)max(0LL, min((long long)S, n - lo));
+  for (int i = tid; i < mx; i += kKryThreads) ex[i] = exph[i];
+  cl.sync();  // every CTA has read beta
+  double s = 0.0;
+  for (int k = tid; k < len; k += kKryThreads) {
+    const double* vk = V + lo + k;
+    double acc = 0.0;
+#pragma unroll 8
+    for (int i = 0; i < mx; ++i) acc += vk[(long long)i * n] * ex[i];
+    const double v = beta * acc;
+    w[lo + k] = v;
+    s += v * v;
+  }
+  s = block_sum(s, red);
+  if (tid == 0) npart = s;
+  cl.sync();
+  if (cl.block_rank() == 0 && tid == 0) {
+    double t = 0.0;
+    for (int q = 0; q < kGsCluster; ++q) t += *cl.map_shared_rank(&npart, q);
+    st->beta = sqrt(t);
+  }
+  cl.sync();  // no CTA leaves while its partial is read
+}
+
+// launch of a kernel on one cluster of kGsCluster CTAs
+template <class... KA, class... A>
+static int launch_gs_cluster(Ctx& c, void (*kernel)(KA...), size_t smem, A... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(kMgsCluster, 1, 1);
+  cfg.gridDim = dim3(kGsCluster, 1, 1);
   cfg.blockDim = dim3(kKryThreads, 1, 1);
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = c.stream;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = kMgsCluster;
+  at[0].val.clusterDim.x = kGsCluster;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  SG_CUDA(cudaLaunchKernelEx(&cfg, kry_mgs_cluster_kernel<E>, V, n, j, Hm, mh, break_tol, st));
+  SG_CUDA(cudaLaunchKernelEx(&cfg, kernel, (KA)args...));
+  count_launch();
   return SINCGPU_OK;
 }
 
@@ -447,14 +467,6 @@ __global__ void __launch_bounds__(kKryThreads) kry_update_kernel(const double* _
   if (threadIdx.x == 0) st->beta = sqrt(s);
 }
 
-// out = scale * in (complex), used to apply timefac after the sigma product
-__global__ void cscale_kernel(const double2* __restrict__ in, double2 s, int nc, double2* __restrict__ out,
-                              const KryState* st) {
-  if (st && st->mbrk) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < nc) out[i] = cmul(s, in[i]);
-}
-
 int pade_expm(Ctx& c, const double* Hm, int mh, int mx, double t, int col, double* exph, double* Efull,
               double* gscratch, int* d_ns) {
   SG_CHECK(mx >= 1 && mx <= kMaxPade, SINCGPU_ERANGE, "Pade order %d outside [1,%d]", mx, kMaxPade);
@@ -485,15 +497,15 @@ int expv_avector(Ctx& c, const double2* v, double2* w, double t, double2 timefac
   SG_CHECK(m > 0 && m < maxdim && m <= kMaxKry, SINCGPU_ERANGE, "Krylov dimension %d outside [1,%lld)", m,
            std::min<long long>(maxdim, kMaxKry + 1));
   const int mh = m + 2;
-  const size_t need = sizeof(double) * ((size_t)(m + 2) * n + (size_t)mh * mh + 128 + 5 * (size_t)mh * mh) +
-                      sizeof(double2) * nc + sizeof(KryState) + 64;
+  const size_t need = sizeof(double) * ((size_t)(m + 2) * n + (size_t)mh * mh + 128 + 6 * (size_t)mh * mh) +
+                      sizeof(KryState) + 64;
   SG_TRY(c.ws_kry.ensure(need));
   double* V = (double*)c.ws_kry.ptr;
   double* Hm = V + (size_t)(m + 2) * n;
   double* exph = Hm + (size_t)mh * mh;
   double* pscr = exph + 128;
-  double2* tmp = (double2*)(pscr + 5 * (size_t)mh * mh);
-  KryState* dst = (KryState*)(tmp + nc);
+  double* Lm = pscr + 5 * (size_t)mh * mh;  // dots of the Krylov vectors (kry_gs_kernel)
+  KryState* dst = (KryState*)(Lm + (size_t)mh * mh);
   int* d_ns = (int*)(dst + 1);
   int nmult = 0;
   const double delta = 1.2, gamma = 0.9, break_tol = 1.0e-7;
@@ -512,7 +524,12 @@ int expv_avector(Ctx& c, const double2* v, double2* w, double t, double2 timefac
   KryState hst{};
   bool have_beta = false;
   ProfScope ps(c, ST_CI);
-  const int cb = ceil_div(nc, 256);
+  // the cluster kernels where a slice of p and v_j fits shared memory, else one CTA
+  const long long S = ((n + kGsCluster - 1) / kGsCluster + 1) / 2 * 2;
+  const bool cluster = c.kry_cluster && S <= kGsSlice;
+  static const cudaError_t attr = cudaFuncSetAttribute(kry_gs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       (int)(sizeof(double) * 2 * kGsSlice));
+  SG_CUDA(attr);
   while (t_now < t_out) {
     ++nstep;
     t_last = t_step;
@@ -522,33 +539,19 @@ int expv_avector(Ctx& c, const double2* v, double2* w, double t, double2 timefac
     SG_LAUNCHED();
     for (int j = 0; j < m; ++j) {
       ++nmult;
-      SG_TRY(ci_sigma(c, (const double2*)(V + (size_t)j * n), tmp, c.nucrepulsion, ez, nucdipz));
-      cscale_kernel<<<cb, 256, 0, c.stream>>>(tmp, timefac, nc, (double2*)(V + (size_t)(j + 1) * n), dst);
-      SG_LAUNCHED();
-      if (n <= kKryThreads)
-        kry_mgs_reg_kernel<1><<<1, kKryThreads, 0, c.stream>>>(V, n, j, Hm, mh, break_tol, dst);
-      else if (n <= 2 * kKryThreads)
-        kry_mgs_reg_kernel<2><<<1, kKryThreads, 0, c.stream>>>(V, n, j, Hm, mh, break_tol, dst);
-      else if (n <= 4 * kKryThreads)
-        kry_mgs_reg_kernel<4><<<1, kKryThreads, 0, c.stream>>>(V, n, j, Hm, mh, break_tol, dst);
-      else if (!c.kry_cluster)
+      SG_TRY(ci_sigma(c, (const double2*)(V + (size_t)j * n), (double2*)(V + (size_t)(j + 1) * n), c.nucrepulsion, ez,
+                      nucdipz, timefac, &dst->mbrk));
+      if (cluster) {
+        SG_TRY(launch_gs_cluster(c, kry_gs_kernel, sizeof(double) * 2 * (size_t)S, V, n, (int)S, j, Hm, mh, Lm,
+                                 break_tol, dst));
+      } else {
         kry_mgs_kernel<<<1, kKryThreads, 0, c.stream>>>(V, n, j, Hm, mh, break_tol, dst);
-      else if (n <= 1LL * kMgsCluster * kKryThreads)
-        SG_TRY(launch_mgs_cluster<1>(c, V, n, j, Hm, mh, break_tol, dst));
-      else if (n <= 2LL * kMgsCluster * kKryThreads)
-        SG_TRY(launch_mgs_cluster<2>(c, V, n, j, Hm, mh, break_tol, dst));
-      else if (n <= 4LL * kMgsCluster * kKryThreads)
-        SG_TRY(launch_mgs_cluster<4>(c, V, n, j, Hm, mh, break_tol, dst));
-      else if (n <= 8LL * kMgsCluster * kKryThreads)
-        SG_TRY(launch_mgs_cluster<8>(c, V, n, j, Hm, mh, break_tol, dst));
-      else
-        kry_mgs_kernel<<<1, kKryThreads, 0, c.stream>>>(V, n, j, Hm, mh, break_tol, dst);
-      SG_LAUNCHED();
+        SG_LAUNCHED();
+      }
     }
     ++nmult;
-    SG_TRY(ci_sigma(c, (const double2*)(V + (size_t)m * n), tmp, c.nucrepulsion, ez, nucdipz));
-    cscale_kernel<<<cb, 256, 0, c.stream>>>(tmp, timefac, nc, (double2*)(V + (size_t)(m + 1) * n), dst);
-    SG_LAUNCHED();
+    SG_TRY(ci_sigma(c, (const double2*)(V + (size_t)m * n), (double2*)(V + (size_t)(m + 1) * n), c.nucrepulsion, ez,
+                    nucdipz, timefac, &dst->mbrk));
     kry_avnorm_kernel<<<1, kKryThreads, 0, c.stream>>>(V + (size_t)(m + 1) * n, n, dst);
     SG_LAUNCHED();
     SG_CUDA(cudaMemcpyAsync(&hst, dst, sizeof(KryState), cudaMemcpyDeviceToHost, c.stream));
@@ -593,8 +596,12 @@ int expv_avector(Ctx& c, const double2* v, double2* w, double t, double2 timefac
       break;
     }
     const int mxu = mbrkdwn + std::max(0, k1 - 1);
-    kry_update_kernel<<<1, kKryThreads, 0, c.stream>>>(V, n, mxu, exph, (double*)w, dst);
-    SG_LAUNCHED();
+    if (cluster) {
+      SG_TRY(launch_gs_cluster(c, kry_update_cluster_kernel, 0, V, n, (int)S, mxu, exph, (double*)w, dst));
+    } else {
+      kry_update_kernel<<<1, kKryThreads, 0, c.stream>>>(V, n, mxu, exph, (double*)w, dst);
+      SG_LAUNCHED();
+    }
     SG_CUDA(cudaMemcpyAsync(&hst, dst, sizeof(KryState), cudaMemcpyDeviceToHost, c.stream));
     SG_CUDA(cudaStreamSynchronize(c.stream));
     t_new = gamma * t_step * std::pow(t_step * tol / err_loc, xm);
