@@ -119,7 +119,7 @@ Ctx::~Ctx() {
   if (stream) cudaStreamSynchronize(stream);
   if (rhs_graph) cudaDeviceSynchronize();
   for (void* p : {(void*)d_kevect, (void*)d_ketile, (void*)d_pot, (void*)d_zdip, (void*)d_tcoul, (void*)d_khat,
-                  (void*)d_roots, (void*)d_khat32, (void*)d_roots32, (void*)d_khT, (void*)d_khT32, (void*)d_khr, (void*)d_khr32, (void*)d_kht, (void*)d_htw})
+                  (void*)d_roots, (void*)d_khat32, (void*)d_roots32, (void*)d_khT, (void*)d_khT32, (void*)d_khr, (void*)d_khr32, (void*)d_kht, (void*)d_htw, (void*)d_count})
     dfree(*this, p);
   ws_fft.release();
   ws_pairs.release();
@@ -313,6 +313,8 @@ static int ctx_common(sincgpu_ctx* h, int numpoints, double spacing, int numspf,
     uint64_t keep = ~0ull;
     cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
   }
+  SG_TRY(dalloc(c, &c.d_count, sizeof(unsigned)));
+  SG_CUDA(cudaMemsetAsync(c.d_count, 0, sizeof(unsigned), c.stream));
   return SINCGPU_OK;
 }
 
@@ -385,7 +387,7 @@ int sincgpu_get_option(sincgpu_ctx* h, const char* name, long long* value) {
     const char* n;
     long long v;
   } opts[] = {{"coul_chunk", c.coul_chunk},       {"coulomb_fp32", c.coul_fp32}, {"contract_tf32", c.contract_tf32},
-              {"coul_half", c.coul_half},         {"coul_tma", c.coul_tma},           {"twoe_tile", c.twoe_tile},    {"orth_fused", c.orth_fused},
+              {"coul_half", c.coul_half}, {"orth_onepass", c.orth_onepass},         {"coul_tma", c.coul_tma},           {"twoe_tile", c.twoe_tile},    {"orth_fused", c.orth_fused},
               {"rhs_overlap", c.rhs_overlap},     {"coul_fused", c.coul_fused},  {"coul_z2", c.coul_z2},
               {"cmf_fp64_last", c.cmf.fp64_last ? 1 : 0}, {"rhs_upload_groups", c.up_groups}, {"kry_cluster", c.kry_cluster}, {"orb_blendq", c.orb_blendq}, {"ke_tf32", c.ke_tf32}, {"tc_kc", c.tc_kc}, {"tc_pipe", c.tc_pipe}, {"twoe_symdiag", c.twoe_symdiag}, {"twoe_dmma", c.twoe_dmma}, {"rp_dmma", c.rp_dmma}};
   for (const auto& o : opts)
@@ -435,6 +437,11 @@ int sincgpu_set_option(sincgpu_ctx* h, const char* name, long long value) {
     SG_CHECK(value >= 1 && value <= Ctx::kUpGroups, SINCGPU_EINVAL, "rhs_upload_groups must be 1..%d",
              Ctx::kUpGroups);
     h->c.up_groups = (int)value;
+    return SINCGPU_OK;
+  }
+  if (!strcmp(name, "orth_onepass")) {
+    SG_CHECK(value == 0 || value == 1, SINCGPU_EINVAL, "orth_onepass must be 0 or 1");
+    h->c.orth_onepass = (int)value;
     return SINCGPU_OK;
   }
   if (!strcmp(name, "orth_fused")) {

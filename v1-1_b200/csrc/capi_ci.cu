@@ -260,9 +260,9 @@ int orbital_rhs_avec_impl(sincgpu_ctx* h, const double* phi, const double* avect
   }
   // reducedpot applies itself to the orbitals in its epilogue where it can
   // (after the kinetic result: ev_join); otherwise actreduced_post applies it
-  double2 *S = nullptr, *T = nullptr, *part = nullptr;
-  int rc = actreduced_temps(c, &S, &T, &part);
-  RpApply ap{P, S, (const double2*)invdenmat, tf, T, c.ev_join, false, P, part};
+  double2 *S = nullptr, *T = nullptr;
+  int rc = actreduced_temps(c, &S, &T);
+  RpApply ap{P, S, (const double2*)invdenmat, tf, T, c.ev_join, false};
   const bool deferred = host_out && twoematel;
   TwoeDefer defer;
   if (rc == SINCGPU_OK)
@@ -270,7 +270,7 @@ int orbital_rhs_avec_impl(sincgpu_ctx* h, const double* phi, const double* avect
                     true, c.ev_ci, twoematel ? c.side : nullptr, &ap, deferred ? &defer : nullptr);
   SG_CUDA(cudaStreamWaitEvent(c.stream, c.ev_join, 0));
   int rc2 = rc == SINCGPU_OK ? actreduced_post(c, P, P, (const double2*)invdenmat, (const double2*)reducedpot, tf,
-                                               1, 1, (double2*)out, ap.done, ap.done)
+                                               1, 1, (double2*)out, ap.done)
                              : rc;
   if (rc2 == SINCGPU_OK && host_out) {
     // the RHS is final: its copy to the host overlaps the deferred twoematel (issued

@@ -217,6 +217,7 @@ struct Ctx {
   int twoe_symdiag = 0;   // 1: multi-tile twoematel computes its diagonal tiles' lower blocks only
   int twoe_tile = 0;      // twoematel tile edge 16R: 0 = least padding, 2..9 = that R
   int orth_fused = 1;     // 1: an orbital Arnoldi step's orthogonalisation in one cooperative launch
+  int orth_onepass = 1;   // 1: the orbital Arnoldi coefficients from one pass of dots, three launches a step
   int kry_cluster = 1;    // 1: A-vector Gram-Schmidt and update on a cluster of CTAs (0: one CTA)
   int orb_blendq = 1;     // 1: the orbital Jacobian reads one blended reduced potential (0: both slots')
   int rhs_overlap = 1;    // 1: the fused orbital-RHS entry runs its CI part and the mix + kinetic
@@ -240,6 +241,7 @@ struct Ctx {
   void* orb_state_h = nullptr;    // page-locked copy of the orbital Krylov state (orbprop.cu)
   size_t orb_state_bytes = 0;
   cudaEvent_t ev_orb_state = nullptr;
+  unsigned* d_count = nullptr;    // arrival counter of kernels whose last CTA finishes a sum (zero between launches)
   Prof prof;
 
   ~Ctx();
@@ -333,10 +335,6 @@ struct RpApply {
   double2* T;
   cudaEvent_t ready;  // S and inv are written on another stream (or nullptr)
   bool done;
-  // when set: also the projector-dot partials part[b][j + n i] = sum over the 64
-  // points of tile b of conj(proj_j) T_i, as dots_kernel forms them (same bits)
-  const double2* proj;
-  double2* part;
 };
 int reduced_pot(Ctx& c, const double* Rpl, const int* h_pa, const int* h_pb, int npair,
                 bool herm, const double2* tally, double2* reducedpot, bool tally_herm = false,
@@ -414,10 +412,9 @@ int actreduced(Ctx& c, const double2* phi, const double2* proj, const double2* d
 int actreduced_pre(Ctx& c, const double2* phi, const double2* denmat, double zfield);
 int actreduced_post(Ctx& c, const double2* phi, const double2* proj, const double2* invdenmat,
                     const double2* redpot, double2 timefac, int dentimeflag, int projflag, double2* out,
-                    bool t_ready = false, bool dots_ready = false);
-// the kinetic result S of actreduced_pre, the apply target T and the projector-dot
-// partials (orbital_dots_scratch(c) blocks of 64 points) in ws_rhs
-int actreduced_temps(Ctx& c, double2** S, double2** T, double2** part = nullptr);
+                    bool t_ready = false);
+// the kinetic result S of actreduced_pre and the apply target T in ws_rhs
+int actreduced_temps(Ctx& c, double2** S, double2** T);
 // actreduced_pre for several density matrices of one phi: the kinetic, potential
 // and field operators act on each orbital alike and so commute with the orbital
 // mixing, KE(phi denmat) = KE(phi) denmat; actreduced_ke forms KE(phi) once (ws_rhs
@@ -441,15 +438,16 @@ int blendq_prepare(Ctx& c, const double2* const* denmat, const double2* const* i
                    const double2* const* redpot, const double* facs);
 int actreduced_blendq(Ctx& c, const double2* x, double2 timefac, double zfield, double2* out);
 int actreduced_mix_ke(Ctx& c, const double2* denmat);
-// D(j,i) = <P_j|T_i> over the grid (split-K, deterministic); part holds
+// D(j,i) = <P_j|T_i> [+ <X_j|O_i>] over the grid (split-K, deterministic); part holds
 // orbital_dots_scratch(c) * nspf^2 partial sums
 int orbital_dots_scratch(const Ctx& c);
-int orbital_dots(Ctx& c, const double2* P, const double2* T, double2* D, double2* part);
+int orbital_dots(Ctx& c, const double2* P, const double2* T, double2* D, double2* part, const double2* X = nullptr,
+                 const double2* O = nullptr);
 // out = in x mat (n x n, column-major)
 int orbital_mix(Ctx& c, const double2* in, const double2* mat, double2* out);
-// out = T - P (M1 + M2) - X D2
-int jac_combine(Ctx& c, const double2* T, const double2* P, const double2* M1, const double2* M2,
-                const double2* X, const double2* D2, double2* out);
+// out = T - P M - X D2
+int jac_combine(Ctx& c, const double2* T, const double2* P, const double2* M, const double2* X, const double2* D2,
+                double2* out);
 // acc = a acc + b in  (acc = b in when `first`)
 int axpby(Ctx& c, double2* acc, const double2* in, double a, double b, long long len, bool first);
 

@@ -260,19 +260,280 @@ __global__ void __launch_bounds__(kLvThreads, 2) lv_arnoldi_orth_kernel(const do
   }
 }
 
+// The orthogonalisation of Arnoldi step j in three launches of any length (option
+// orth_onepass): the coefficients of the modified Gram-Schmidt from one pass of dots.
+// With r_i = <v_i, p> and L_ik = <v_i, v_k> (k < i; rounding level), the sequential
+// projections' h solve (I + L) h = r, so h = r - L r up to L^2, which is far below
+// rounding.  Row j of L is summed in the same pass (v_j is a row already) and kept.
+//   lv_dots_all: r and row j of L, eight rows of V at a time in registers; the last CTA
+//                adds the partials in a fixed order and forms h
+//   lv_project:  p -= sum_i h_i v_i and |p|^2; the last CTA sets h(j+1,j) and breakdown
+//   lv_scale:    p /= h(j+1,j)
+// Bound by HBM or L2: V is read twice, 32 nv (j + 3) bytes.  The one cooperative launch
+// above reads V once but waits at j + 2 grid barriers, each with a block sum on both
+// sides; where p fits the registers, lv_orth_onepass_kernel does these three passes in
+// one launch with two barriers: 48 -> 35 us a step at 41^3 / 10 orbitals, ten vectors
+// (cold caches; three launches took 47).
+constexpr int kRows = 8;
+
+// adds this CTA to *count; true in the last one (which resets it for the next launch)
+__device__ __forceinline__ bool lv_last_cta(unsigned* count, unsigned* sh) {
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    *sh = atomicAdd(count, 1u) == gridDim.x - 1;
+    if (*sh) *count = 0;
+  }
+  __syncthreads();
+  if (*sh) __threadfence();
+  return *sh != 0;
+}
+
+// totals of the 2 (j + 1) dots over the CTAs' partials in a fixed order, row j of L (to
+// Lm when `keep`) and the coefficients h; one CTA
+__device__ __forceinline__ void lv_coefficients(const double* part, int j, double* tot, double* h, double* Lm, int mh,
+                                                bool keep) {
+  constexpr int U = (kLvBlocks + 31) / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int e = warp; e < 2 * (j + 1); e += kLvThreads / 32) {
+    double v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = lane + 32 * u < kLvBlocks ? __ldcg(part + (long long)e * kLvBlocks + lane + 32 * u) : 0.0;
+    double s = 0.0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) s += v[u];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) {
+      tot[e] = s;
+      if (keep && (e & 1) && e / 2 < j) Lm[(long long)j * mh + e / 2] = s;
+    }
+  }
+  __syncthreads();
+  for (int i = warp; i <= j; i += kLvThreads / 32) {
+    double a = 0.0;
+    for (int k = lane; k < i; k += 32) a = fma(i < j ? Lm[(long long)i * mh + k] : tot[2 * k + 1], tot[2 * k], a);
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+    if (lane == 0) h[i] = tot[2 * i] - a;
+  }
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(kLvThreads, 2) lv_dots_all_kernel(const double2* __restrict__ V,
+                                                                     const double2* __restrict__ p, long long nv, int j,
+                                                                     double* __restrict__ part, double* __restrict__ Hm,
+                                                                     int mh, double* __restrict__ Lm,
+                                                                     const OrbKryState* __restrict__ st,
+                                                                     unsigned* __restrict__ count) {
+  __shared__ double red[kLvThreads / 32][2 * kRows];
+  __shared__ double tot[256], h[128];
+  __shared__ unsigned last;
+  if (st->mbrk) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const double2* vj = V + (long long)j * nv;
+  for (int c0 = 0; c0 <= j; c0 += kRows) {
+    double r[kRows], g[kRows];
+#pragma unroll
+    for (int q = 0; q < kRows; ++q) r[q] = g[q] = 0.0;
+    for (long long k = blockIdx.x * (long long)kLvThreads + tid; k < nv; k += (long long)gridDim.x * kLvThreads) {
+      const double2 x = p[k], y = vj[k];
+      double2 v[kRows];
+#pragma unroll
+      for (int q = 0; q < kRows; ++q) v[q] = c0 + q <= j ? V[(long long)(c0 + q) * nv + k] : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int q = 0; q < kRows; ++q) {
+        r[q] = fma(v[q].y, x.y, fma(v[q].x, x.x, r[q]));
+        g[q] = fma(v[q].y, y.y, fma(v[q].x, y.x, g[q]));
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kRows; ++q)
+      for (int o = 16; o > 0; o >>= 1) {
+        r[q] += __shfl_down_sync(0xffffffffu, r[q], o);
+        g[q] += __shfl_down_sync(0xffffffffu, g[q], o);
+      }
+    __syncthreads();  // the previous rows' sums are read
+    if (lane == 0)
+#pragma unroll
+      for (int q = 0; q < kRows; ++q) {
+        red[warp][2 * q] = r[q];
+        red[warp][2 * q + 1] = g[q];
+      }
+    __syncthreads();
+    if (tid < 2 * kRows && c0 + tid / 2 <= j) {
+      double s = 0.0;
+#pragma unroll
+      for (int w = 0; w < kLvThreads / 32; ++w) s += red[w][tid];
+      part[(long long)(2 * c0 + tid) * kLvBlocks + blockIdx.x] = s;
+    }
+  }
+  if (!lv_last_cta(count, &last)) return;
+  lv_coefficients(part, j, tot, h, Lm, mh, true);
+  if (tid <= j) Hm[(long long)j * mh + tid] = h[tid];
+}
+
+// The same step in one cooperative launch (nv <= E kLvBlocks kLvThreads): p stays in
+// registers, grid barriers after the dots and after the norm; every CTA adds the
+// partials itself, in the same order.
+template <int E>
+__global__ void __launch_bounds__(kLvThreads, 2) lv_orth_onepass_kernel(const double2* __restrict__ V, double2* p,
+                                                                         long long nv, int j, double* part, double* partn,
+                                                                         double* __restrict__ Hm, int mh, double* Lm,
+                                                                         double break_tol, OrbKryState* st,
+                                                                         unsigned* bar) {
+  constexpr int R = 4;  // rows of V in registers at a time
+  __shared__ double rsum[kLvThreads / 32][2 * R], red[33];
+  __shared__ double tot[256], h[128];
+  __shared__ int ok;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const long long stride = (long long)gridDim.x * kLvThreads, k0 = blockIdx.x * (long long)kLvThreads + tid;
+  const double2* vj = V + (long long)j * nv;
+  const double2 zero = make_double2(0.0, 0.0);
+  double2 x[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) x[e] = k0 + e * stride < nv ? p[k0 + e * stride] : zero;
+  for (int c0 = 0; c0 <= j; c0 += R) {
+    double r[R], g[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) r[q] = g[q] = 0.0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const long long k = k0 + e * stride;
+      const double2 y = k < nv ? vj[k] : zero;
+      double2 v[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[q] = c0 + q <= j && k < nv ? V[(long long)(c0 + q) * nv + k] : zero;
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        r[q] = fma(v[q].y, x[e].y, fma(v[q].x, x[e].x, r[q]));
+        g[q] = fma(v[q].y, y.y, fma(v[q].x, y.x, g[q]));
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < R; ++q)
+      for (int o = 16; o > 0; o >>= 1) {
+        r[q] += __shfl_down_sync(0xffffffffu, r[q], o);
+        g[q] += __shfl_down_sync(0xffffffffu, g[q], o);
+      }
+    __syncthreads();  // the previous rows' sums are read
+    if (lane == 0)
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        rsum[warp][2 * q] = r[q];
+        rsum[warp][2 * q + 1] = g[q];
+      }
+    __syncthreads();
+    if (tid < 2 * R && c0 + tid / 2 <= j) {
+      double s = 0.0;
+#pragma unroll
+      for (int w = 0; w < kLvThreads / 32; ++w) s += rsum[w][tid];
+      part[(long long)(2 * c0 + tid) * kLvBlocks + blockIdx.x] = s;
+    }
+  }
+  if (!grid_barrier(bar, st, &ok)) return;
+  lv_coefficients(part, j, tot, h, Lm, mh, blockIdx.x == 0);
+  if (blockIdx.x == 0 && tid <= j) Hm[(long long)j * mh + tid] = h[tid];
+  double s = 0.0;
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const long long k = k0 + e * stride;
+    if (k >= nv) continue;
+    for (int c0 = 0; c0 <= j; c0 += R) {
+      double2 v[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[q] = c0 + q <= j ? V[(long long)(c0 + q) * nv + k] : zero;
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const double c = c0 + q <= j ? h[c0 + q] : 0.0;
+        x[e].x = fma(-c, v[q].x, x[e].x);
+        x[e].y = fma(-c, v[q].y, x[e].y);
+      }
+    }
+    s = fma(x[e].x, x[e].x, s);
+    s = fma(x[e].y, x[e].y, s);
+  }
+  s = lv_block_sum(s, red);
+  if (tid == 0) partn[blockIdx.x] = s;
+  if (!grid_barrier(bar, st, &ok)) return;
+  const double hn = sqrt(lv_total_l2(partn, red));
+  const bool brk = hn <= break_tol;
+  if (blockIdx.x == 0 && tid == 0) {
+    st->hlast = hn;
+    if (brk) st->mbrk = j + 1;
+    else Hm[(long long)j * mh + j + 1] = hn;
+  }
+  const double inv = 1.0 / hn;
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const long long k = k0 + e * stride;
+    if (k < nv) p[k] = brk ? x[e] : make_double2(x[e].x * inv, x[e].y * inv);
+  }
+}
+
+__global__ void __launch_bounds__(kLvThreads, 2) lv_project_kernel(const double2* __restrict__ V, double2* __restrict__ p,
+                                                                    long long nv, int j, double* __restrict__ part,
+                                                                    double* __restrict__ Hm, int mh, double break_tol,
+                                                                    OrbKryState* __restrict__ st,
+                                                                    unsigned* __restrict__ count) {
+  __shared__ double red[33], h[128];
+  __shared__ unsigned last;
+  if (st->mbrk) return;
+  const int tid = threadIdx.x;
+  if (tid <= j) h[tid] = Hm[(long long)j * mh + tid];
+  __syncthreads();
+  double s = 0.0;
+  for (long long k = blockIdx.x * (long long)kLvThreads + tid; k < nv; k += (long long)gridDim.x * kLvThreads) {
+    double2 x = p[k];
+    for (int c0 = 0; c0 <= j; c0 += kRows) {
+      double2 v[kRows];
+#pragma unroll
+      for (int q = 0; q < kRows; ++q) v[q] = c0 + q <= j ? V[(long long)(c0 + q) * nv + k] : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int q = 0; q < kRows; ++q) {
+        const double c = c0 + q <= j ? h[c0 + q] : 0.0;
+        x.x = fma(-c, v[q].x, x.x);
+        x.y = fma(-c, v[q].y, x.y);
+      }
+    }
+    p[k] = x;
+    s = fma(x.x, x.x, s);
+    s = fma(x.y, x.y, s);
+  }
+  s = lv_block_sum(s, red);
+  if (tid == 0) part[blockIdx.x] = s;
+  if (!lv_last_cta(count, &last)) return;
+  const double hn = sqrt(lv_total_l2(part, red));
+  if (tid == 0) {
+    st->hlast = hn;
+    if (hn <= break_tol) st->mbrk = j + 1;
+    else Hm[(long long)j * mh + j + 1] = hn;
+  }
+}
+
+__global__ void __launch_bounds__(kLvThreads) lv_scale_kernel(double2* __restrict__ p, long long nv,
+                                                              const OrbKryState* __restrict__ st) {
+  if (st->mbrk) return;
+  const double inv = 1.0 / st->hlast;
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nv;
+       k += (long long)gridDim.x * blockDim.x) {
+    const double2 x = p[k];
+    p[k] = make_double2(x.x * inv, x.y * inv);
+  }
+}
+
 constexpr int kOrthE = 5;  // register-resident elements per thread of the one-launch orthogonalisation
 
-// whether all kLvBlocks CTAs of lv_arnoldi_orth_kernel fit on the device at once
-// (the cooperative launch needs it); evaluated once per process
+// whether all kLvBlocks CTAs of the one-launch orthogonalisations fit on the device at
+// once (a cooperative launch needs it); evaluated once per process
 static bool orth_fits() {
   static const bool fits = [] {
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return false;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lv_arnoldi_orth_kernel<kOrthE>, kLvThreads, 0) !=
-        cudaSuccess)
-      return false;
-    return (long long)per_sm * sms >= kLvBlocks;
+    for (const void* k : {(const void*)lv_arnoldi_orth_kernel<kOrthE>, (const void*)lv_orth_onepass_kernel<kOrthE>}) {
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kLvThreads, 0) != cudaSuccess) return false;
+      if ((long long)per_sm * sms < kLvBlocks) return false;
+    }
+    return true;
   }();
   return fits;
 }
@@ -372,11 +633,12 @@ namespace {
 // device scratch of one orbital propagation
 struct OrbWork {
   double2 *V, *jv, *jvo, *u, *w, *T, *tmp, *dpart;
-  double2 *D2, *M1, *M2, *ovl, *smh;
+  double2 *D2, *M1, *ovl, *smh;
   double *part0, *part1, *Hm, *exph, *Efull, *pscratch, *err;
+  double *gpart, *Lm;  // lv_dots_all_kernel's partials and the dots of the Krylov vectors
   OrbKryState* st;
   int* ns;
-  unsigned* gbar;  // lv_arnoldi_orth_kernel's grid barrier (count, generation)
+  unsigned* gbar;  // lv_arnoldi_orth_kernel's grid barrier (count, generation), lv_last_cta's count
   bool blendq = false;  // the unprojected blends read the prepared Q and M (blendq_prepare)
 };
 
@@ -389,8 +651,9 @@ int orb_work(Ctx& c, int m, OrbWork& o) {
   const size_t vb = sizeof(double2) * (size_t)nv;
   const size_t dpart = sizeof(double2) * (size_t)orbital_dots_scratch(c) * nn;
   const size_t mat = sizeof(double2) * nn;
-  size_t need = al256(vb) * ((size_t)m + 2 + 6) + al256(dpart) + 5 * al256(mat) +
-                2 * al256(sizeof(double) * kLvBlocks) + al256(sizeof(double) * mh * mh) +
+  size_t need = al256(vb) * ((size_t)m + 2 + 6) + al256(dpart) + 4 * al256(mat) +
+                2 * al256(sizeof(double) * kLvBlocks) + 2 * al256(sizeof(double) * mh * mh) +
+                al256(sizeof(double) * 2 * (m + 1) * kLvBlocks) +
                 al256(sizeof(double) * 130) + al256(sizeof(double) * kMaxPadeOrb * kMaxPadeOrb) +
                 al256(sizeof(double) * 5 * kMaxPadeOrb * kMaxPadeOrb) + 4 * 256;
   SG_TRY(c.ws_orb.ensure(need));
@@ -410,19 +673,20 @@ int orb_work(Ctx& c, int m, OrbWork& o) {
   o.dpart = (double2*)take(dpart);
   o.D2 = (double2*)take(mat);
   o.M1 = (double2*)take(mat);
-  o.M2 = (double2*)take(mat);
   o.ovl = (double2*)take(mat);
   o.smh = (double2*)take(mat);
   o.part0 = (double*)take(sizeof(double) * kLvBlocks);
   o.part1 = (double*)take(sizeof(double) * kLvBlocks);
   o.Hm = (double*)take(sizeof(double) * mh * mh);
+  o.Lm = (double*)take(sizeof(double) * mh * mh);
+  o.gpart = (double*)take(sizeof(double) * 2 * (m + 1) * kLvBlocks);
   o.exph = (double*)take(sizeof(double) * 130);
   o.Efull = (double*)take(sizeof(double) * kMaxPadeOrb * kMaxPadeOrb);
   o.pscratch = (double*)take(sizeof(double) * 5 * kMaxPadeOrb * kMaxPadeOrb);
   o.err = (double*)take(sizeof(double));
   o.st = (OrbKryState*)take(sizeof(OrbKryState));
   o.ns = (int*)take(sizeof(int));
-  o.gbar = (unsigned*)take(2 * sizeof(unsigned));
+  o.gbar = (unsigned*)take(3 * sizeof(unsigned));
   return SINCGPU_OK;
 }
 
@@ -467,9 +731,8 @@ int blend_actreduced(Ctx& c, const double2* x, const double2* proj, const MeanFi
 int jacoperate(Ctx& c, OrbWork& o, const double2* x, const MeanFieldSlot* slots, const double* facs, int nslot,
                double2 timefac, double ez, double2* y) {
   SG_TRY(blend_actreduced(c, x, nullptr, slots, facs, nslot, timefac, ez, o.tmp, o.T, o.blendq));
-  SG_TRY(orbital_dots(c, o.jv, o.T, o.M1, o.dpart));   // <jacvect|T>
-  SG_TRY(orbital_dots(c, x, o.jvo, o.M2, o.dpart));    // <x|jacvectout>
-  return jac_combine(c, o.T, o.jv, o.M1, o.M2, x, o.D2, y);
+  SG_TRY(orbital_dots(c, o.jv, o.T, o.M1, o.dpart, x, o.jvo));  // <jacvect|T> + <x|jacvectout>
+  return jac_combine(c, o.T, o.jv, o.M1, x, o.D2, y);
 }
 
 double fortran_nint(double x) { return x >= 0 ? std::floor(x + 0.5) : -std::floor(-x + 0.5); }
@@ -559,8 +822,9 @@ int expospfprop(Ctx& c, double2* phi, const MeanFieldSlot* slots, double tin, do
   bool w_zero = true;
   SG_CUDA(cudaMemsetAsync(o.w, 0, sizeof(double2) * nv, c.stream));
   const int lvg = kLvBlocks;
-  const bool orth_fused = c.orth_fused && nv <= (long long)kOrthE * lvg * kLvThreads && orth_fits();
-  SG_CUDA(cudaMemsetAsync(o.gbar, 0, 2 * sizeof(unsigned), c.stream));
+  const bool one_launch = nv <= (long long)kOrthE * lvg * kLvThreads && orth_fits();
+  const bool orth_fused = c.orth_fused && one_launch;
+  SG_CUDA(cudaMemsetAsync(o.gbar, 0, 3 * sizeof(unsigned), c.stream));
   SG_CUDA(cudaMemsetAsync(o.st, 0, sizeof(OrbKryState), c.stream));
   const int ub = std::min<long long>(ceil_div(nv, 256), 148 * 8);
   OrbKryState hst{};
@@ -600,7 +864,28 @@ int expospfprop(Ctx& c, double2* phi, const MeanFieldSlot* slots, double tin, do
       ++nmult;
       double2* p = o.V + (size_t)(j + 1) * nv;
       if (!have_next) SG_TRY(jacoperate(c, o, o.V + (size_t)j * nv, slots, facs, nslot, timefac, ez, p));
-      if (orth_fused) {
+      if (c.orth_onepass && one_launch) {
+        const double2* Vc = o.V;
+        double *P0 = o.gpart, *P1 = o.part0, *H = o.Hm, *Lm = o.Lm;
+        OrbKryState* S = o.st;
+        unsigned* B = o.gbar;
+        int jj = j, mhh = mh;
+        long long nvv = nv;
+        double bt = break_tol;
+        void* args[] = {(void*)&Vc, (void*)&p,   (void*)&nvv, (void*)&jj, (void*)&P0, (void*)&P1,
+                        (void*)&H,  (void*)&mhh, (void*)&Lm,  (void*)&bt, (void*)&S,  (void*)&B};
+        SG_CUDA(cudaLaunchCooperativeKernel((const void*)lv_orth_onepass_kernel<kOrthE>, dim3(lvg), dim3(kLvThreads),
+                                            args, 0, c.stream));
+        count_launch();
+      } else if (c.orth_onepass) {
+        lv_dots_all_kernel<<<lvg, kLvThreads, 0, c.stream>>>(o.V, p, nv, j, o.gpart, o.Hm, mh, o.Lm, o.st, o.gbar + 2);
+        SG_LAUNCHED();
+        lv_project_kernel<<<lvg, kLvThreads, 0, c.stream>>>(o.V, p, nv, j, o.part0, o.Hm, mh, break_tol, o.st,
+                                                            o.gbar + 2);
+        SG_LAUNCHED();
+        lv_scale_kernel<<<lvg, kLvThreads, 0, c.stream>>>(p, nv, o.st);
+        SG_LAUNCHED();
+      } else if (orth_fused) {
         const double2* Vc = o.V;
         double *P0 = o.part0, *P1 = o.part1, *H = o.Hm;
         OrbKryState* S = o.st;

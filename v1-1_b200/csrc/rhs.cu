@@ -5,11 +5,11 @@
 //   S     += sum_k reducedpot(:,k,i) phi_k                  (line 763, mult_reducedpot)
 //   S      = timefac * S x invdenmat        (dentimeflag)   (lines 788-790)
 //   out    = S - proj x <proj|S>            (projflag)      (lines 806-807, project00)
-// Kernels: mix (pointwise n x n), KE (ke.cu, fused pot/pulse), reducedpot apply +
-// invdenmat mix (one pass over reducedpot, the dominant HBM stream), projector
-// dots (split-K, deterministic), projector subtraction.
+// Kernels: mix and projector subtraction (lin_kernel, FP64 tensor cores), KE (ke.cu,
+// fused pot/pulse), reducedpot apply + invdenmat mix (one pass over reducedpot, the
+// dominant HBM stream), projector dots (FP64 tensor cores, split-K, deterministic).
 //
-// The per-point kernels work on tiles of 32 consecutive grid points (one per
+// The other per-point kernels work on tiles of 32 consecutive grid points (one per
 // lane) by all orbitals: each warp handles a subset of output orbitals, reads
 // every (orbital, tile) row as one coalesced 512-byte segment, and the small
 // per-point vectors (phi, the partial sums) and n x n matrices sit in shared
@@ -23,25 +23,89 @@ constexpr int TXO = 32;          // grid points per tile (lanes)
 constexpr int kMaxOrbRhs = 32;   // largest orbital count of these kernels
 constexpr int kRhsSmemMax = 64 * 1024;
 
-// out(x,i) = sum_j in(x,j) mat(j,i)   (column-major n x n complex mat)
-__global__ void __launch_bounds__(TXO * kMaxOrbRhs) mix_kernel(const double2* __restrict__ in,
-                                                        const double2* __restrict__ mat, int n, long long G,
-                                                        double2* __restrict__ out) {
-  extern __shared__ double2 rsm[];
-  double2* sm = rsm;            // n*n
-  double2* tin = rsm + n * n;   // n x TXO
-  const int lx = threadIdx.x, ty = threadIdx.y, tid = ty * TXO + lx;
-  for (int e = tid; e < n * n; e += TXO * blockDim.y) sm[e] = mat[e];
-  const long long x = blockIdx.x * (long long)TXO + lx;
-  const bool ok = x < G;
-  for (int j = ty; j < n; j += blockDim.y) tin[j * TXO + lx] = ok ? in[(long long)j * G + x] : make_double2(0.0, 0.0);
-  __syncthreads();
-  if (!ok) return;
-  for (int i = ty; i < n; i += blockDim.y) {
-    double2 acc = make_double2(0.0, 0.0);
-    for (int j = 0; j < n; ++j) cfma(acc, tin[j * TXO + lx], sm[j + n * i]);
-    out[(long long)i * G + x] = acc;
+__device__ __forceinline__ void dmma_884(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+
+// out(x,i) = [base(x,i)] + sgn sum_s sum_j src_s(x,j) mat_s(j,i), s < NS (column-major n x n
+// complex matrices): the mix with denmat or an overlap's root, the projection and the
+// Jacobian's combination, as products of a G x 2n by a 2n x 2n real matrix on the FP64
+// tensor cores (complex entries as 2 x 2 real blocks).  A warp owns LMT x 8 points and all
+// 2n columns (NT fragments of 8 = 4 orbitals).  Fragments of src come straight from
+// global memory (lanes = 8 points x (2 orbitals, re/im): whole lines), all of a source
+// in flight together; the matrices sit in shared memory in fragment order, read once
+// per warp.  Bound by HBM: 16 G n (NS + 1 or 2) bytes, 3.4 to 7 us at 41^3 / 10 orbitals.
+// The per-point form (one lane per point, matrix and tile read from shared memory for
+// every product) was bound by shared-memory reads: mix 11.3 -> 8.5, projection 12.6 ->
+// 8.5, Jacobian's combination 18.3 -> 14.2 us there (cold caches).
+constexpr int LMT = 2;            // fragments of 8 points per warp
+constexpr int kLinWarps = 8;
+template <int NS, int NT>
+__global__ void __launch_bounds__(32 * kLinWarps) lin_kernel(const double2* __restrict__ base,
+                                                             const double2* __restrict__ src0,
+                                                             const double2* __restrict__ mat0,
+                                                             const double2* __restrict__ src1,
+                                                             const double2* __restrict__ mat1, double sgn, int n,
+                                                             long long G, double2* __restrict__ out) {
+  constexpr int KS = 2 * NT;  // K steps of 4 = 2 orbitals
+  extern __shared__ double lsm[];  // [NS][KS][NT][32]
+  const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  for (int e = tid; e < NS * KS * NT * 32; e += blockDim.x) {
+    const int l = e & 31, nt = (e >> 5) % NT, ks = (e >> 5) / NT % KS, s = (e >> 5) / (NT * KS);
+    const int j = 2 * ks + ((l & 3) >> 1), i = 4 * nt + (l >> 3), cj = l & 1, ci = (l >> 2) & 1;
+    double v = 0.0;
+    if (j < n && i < n) {
+      const double2 m = (s ? mat1 : mat0)[j + n * i];
+      v = cj == ci ? m.x : (cj ? -m.y : m.y);
+    }
+    lsm[e] = sgn * v;
   }
+  const long long x0 = (blockIdx.x * (long long)kLinWarps + (tid >> 5)) * (8 * LMT) + g;
+  double acc[LMT][NT][2];
+#pragma unroll
+  for (int m = 0; m < LMT; ++m)
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      const long long x = x0 + 8 * m;
+      const int i = 4 * nt + t;
+      const double2 b = base && x < G && i < n ? base[(long long)i * G + x] : make_double2(0.0, 0.0);
+      acc[m][nt][0] = b.x;
+      acc[m][nt][1] = b.y;
+    }
+  double a[KS][LMT];
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    const double* src = reinterpret_cast<const double*>(s ? src1 : src0) + (t & 1);
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+      for (int m = 0; m < LMT; ++m) {
+        const long long x = x0 + 8 * m;
+        const int j = 2 * ks + (t >> 1);
+        a[ks][m] = j < n && x < G ? src[2 * ((long long)j * G + x)] : 0.0;
+      }
+    if (s == 0) __syncthreads();  // the matrices
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+      if (2 * ks >= n) break;
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        const double b = lsm[((s * KS + ks) * NT + nt) * 32 + lane];
+#pragma unroll
+        for (int m = 0; m < LMT; ++m) dmma_884(acc[m][nt], a[ks][m], b);
+      }
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < LMT; ++m)
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      const long long x = x0 + 8 * m;
+      const int i = 4 * nt + t;
+      if (x < G && i < n) out[(long long)i * G + x] = make_double2(acc[m][nt][0], acc[m][nt][1]);
+    }
 }
 
 // s_i = acc(x,i) + sum_k V(x,k,i) phi_k(x) over i in [i0, i0+ni); then, when
@@ -86,9 +150,9 @@ __global__ void __launch_bounds__(TXO * kMaxOrbRhs) redpot_kernel(const double2*
 
 // actreduced blended over two mean-field slots without projection (the orbital
 // Jacobian): out = f0 A_0 + f1 A_1 with A_s = timefac ((Y D_s + V_s . x) I_s) and
-// Y = KE(x) (+ potential and field), per point in one pass: mix_kernel,
-// redpot_kernel (dentime) and axpby_kernel's arithmetic in their order, so the
-// same bits as those launches, without the per-slot temporaries.
+// Y = KE(x) (+ potential and field), per point in one pass: the mix,
+// redpot_kernel (dentime) and axpby_kernel in one, without the
+// per-slot temporaries.
 __global__ void __launch_bounds__(TXO * kMaxOrbRhs) blend2_kernel(
     const double2* __restrict__ xin, const double2* __restrict__ Y, const double2* __restrict__ V0,
     const double2* __restrict__ V1, const double2* __restrict__ D0, const double2* __restrict__ D1,
@@ -219,9 +283,8 @@ __global__ void __launch_bounds__(TXO * kMaxOrbRhs) blendq_apply_kernel(
 
 // partial[blk][j + n*i] = sum_{x in blk} conj(P_j(x)) T_i(x); block blk covers
 // DCH consecutive points, warp w the rows j = w, w + (warps per block), ...
-// BL points per block: 64 (DCH) where the reducedpot GEMM's epilogue forms the same
-// partials for its 64-point tiles, 256 for the orbital Jacobian's dots (eight terms
-// per lane before the shuffle tree, a quarter of the partials to reduce)
+// (beyond 16 orbitals).  BL points per block: 256 (eight terms per lane before the shuffle
+// tree, a quarter of the partials to reduce) where they fit shared memory, else 64
 constexpr int DCH = 64;
 template <int BL>
 __global__ void __launch_bounds__(TXO * kMaxOrbRhs) dots_kernel(const double2* __restrict__ Pm,
@@ -290,63 +353,116 @@ __global__ void __launch_bounds__(128) dots_reduce_kernel(const double2* __restr
   if (threadIdx.x == 0) D[e] = red[0];
 }
 
-// out(x,i) = T(x,i) - sum_j P_j(x) D(j,i)
-__global__ void __launch_bounds__(TXO * kMaxOrbRhs) project_kernel(const double2* __restrict__ Tm,
-                                                            const double2* __restrict__ Pm,
-                                                            const double2* __restrict__ D, int n, long long G,
-                                                            double2* __restrict__ out) {
-  extern __shared__ double2 rsm[];
-  double2* sd = rsm;            // n*n
-  double2* sp = rsm + n * n;    // n x TXO
-  const int lx = threadIdx.x, ty = threadIdx.y, tid = ty * TXO + lx;
-  for (int e = tid; e < n * n; e += TXO * blockDim.y) sd[e] = D[e];
-  const long long x = blockIdx.x * (long long)TXO + lx;
-  const bool ok = x < G;
-  for (int j = ty; j < n; j += blockDim.y) sp[j * TXO + lx] = ok ? Pm[(long long)j * G + x] : make_double2(0.0, 0.0);
-  __syncthreads();
-  if (!ok) return;
-  for (int i = ty; i < n; i += blockDim.y) {
-    double2 a = make_double2(0.0, 0.0);
-    for (int j = 0; j < n; ++j) cfma(a, sp[j * TXO + lx], sd[j + n * i]);
-    out[(long long)i * G + x] = csub(Tm[(long long)i * G + x], a);
+// D(j,i) = sum_x conj(P_j(x)) T_i(x) [+ conj(X_j(x)) O_i(x)] on the FP64 tensor cores: the
+// 2n x 2n real products of the rows (orbital, re/im), K = the points.  A warp sums a
+// run of points into all NT x NT fragments (n <= 4 NT orbitals), fragments straight from
+// global memory (lanes = 4 points x (4 orbitals, re/im)); the CTA adds its warps' sums in
+// order, and the last CTA to finish adds the CTAs' partials in a fixed order
+// (deterministic).  Bound by HBM: 32 G n bytes a pair, 3.4 us at 41^3 / 10 orbitals, and
+// by the latency of the two sums at its end.  dots_kernel below spends ten shuffles on
+// each of its n^2 sums per 64 or 256 points: with its reduction 24.5 -> 13.5 us there, the
+// Jacobian's two products of one launch instead of four 34 -> 17.8 us (cold caches).
+constexpr int kDotWarps = 16, kDotBlocks = 148;
+constexpr int dot_points(int nt) { return nt <= 3 ? 16 : 8; }  // points per step of a warp (by registers)
+template <int NT>
+__global__ void __launch_bounds__(32 * kDotWarps) dots_mma_kernel(const double2* __restrict__ P,
+                                                                  const double2* __restrict__ T,
+                                                                  const double2* __restrict__ X,
+                                                                  const double2* __restrict__ O, int n, long long G,
+                                                                  double2* __restrict__ part, double2* __restrict__ D,
+                                                                  unsigned* __restrict__ count) {
+  extern __shared__ double dsm[];  // [kDotWarps][NT * NT * 64]
+  __shared__ unsigned last;
+  constexpr int NE = NT * NT * 64, kDotPts = dot_points(NT);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const long long W = (long long)gridDim.x * kDotWarps, w = (long long)warp * gridDim.x + blockIdx.x;
+  double acc[NT][NT][2];
+#pragma unroll
+  for (int a = 0; a < NT; ++a)
+#pragma unroll
+    for (int b = 0; b < NT; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+  for (int s = 0; s < (X ? 2 : 1); ++s) {
+    const double* L = reinterpret_cast<const double*>(s ? X : P) + (g & 1);
+    const double* R = reinterpret_cast<const double*>(s ? O : T) + (g & 1);
+    for (long long x0 = w * kDotPts; x0 < G; x0 += W * kDotPts) {
+      double l[NT][kDotPts / 4], r[NT][kDotPts / 4];
+#pragma unroll
+      for (int q = 0; q < kDotPts / 4; ++q)
+#pragma unroll
+        for (int a = 0; a < NT; ++a) {
+          const int j = 4 * a + (g >> 1);
+          const long long x = x0 + 4 * q + t;
+          const bool ok = j < n && x < G;
+          l[a][q] = ok ? L[2 * ((long long)j * G + x)] : 0.0;
+          r[a][q] = ok ? R[2 * ((long long)j * G + x)] : 0.0;
+        }
+#pragma unroll
+      for (int q = 0; q < kDotPts / 4; ++q)
+#pragma unroll
+        for (int a = 0; a < NT; ++a)
+#pragma unroll
+          for (int b = 0; b < NT; ++b) dmma_884(acc[a][b], l[a][q], r[b][q]);
+    }
   }
+#pragma unroll
+  for (int a = 0; a < NT; ++a)
+#pragma unroll
+    for (int b = 0; b < NT; ++b) {  // row 8 a + g, columns 8 b + 2 t, + 1
+      double* o = dsm + warp * NE + (8 * a + g) * (8 * NT) + 8 * b + 2 * t;
+      o[0] = acc[a][b][0];
+      o[1] = acc[a][b][1];
+    }
+  __syncthreads();
+  for (int e = tid; e < NE; e += blockDim.x) {
+    double v = 0.0;
+#pragma unroll
+    for (int q = 0; q < kDotWarps; ++q) v += dsm[q * NE + e];
+    dsm[e] = v;  // element e of warp 0's block is read by this thread alone
+  }
+  __syncthreads();
+  const int nn = n * n;
+  for (int e = tid; e < nn; e += blockDim.x) {
+    const int j = e % n, i = e / n;
+    const double* c0 = dsm + (2 * j) * (8 * NT) + 2 * i;  // (re, .) row
+    const double* c1 = c0 + 8 * NT;                       // (im, .) row
+    part[(long long)blockIdx.x * nn + e] = make_double2(c0[0] + c1[1], c0[1] - c1[0]);
+  }
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) last = atomicAdd(count, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  // thread (c, e) sums the c-th share of the CTAs for element e (consecutive threads,
+  // consecutive elements; eight loads in flight), then the shares are added in order
+  const int nc = max(1, (int)blockDim.x / nn), per = ((int)gridDim.x + nc - 1) / nc;
+  double2* sh = reinterpret_cast<double2*>(dsm);  // [nc][nn]
+  for (int q = tid; q < nc * nn; q += blockDim.x) {
+    const int cc = q / nn, e = q - cc * nn, b1 = min((int)gridDim.x, (cc + 1) * per);
+    double2 v = make_double2(0.0, 0.0);
+    for (int b = cc * per; b < b1; b += 8) {
+      double2 w[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        w[u] = b + u < b1 ? __ldcg(part + (long long)(b + u) * nn + e) : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v = cadd(v, w[u]);
+    }
+    sh[q] = v;
+  }
+  __syncthreads();
+  for (int e = tid; e < nn; e += blockDim.x) {
+    double2 v = sh[e];
+    for (int cc = 1; cc < nc; ++cc) v = cadd(v, sh[cc * nn + e]);
+    D[e] = v;
+  }
+  if (tid == 0) *count = 0;  // for the next launch on this stream
 }
 
-// out(x,i) = T(x,i) - sum_j P_j(x) (M1(j,i) + M2(j,i)) - sum_j X_j(x) D2(j,i)
-// (the projector and projector-derivative terms of the orbital Jacobian)
-__global__ void __launch_bounds__(TXO * kMaxOrbRhs) jac_combine_kernel(const double2* __restrict__ Tm,
-                                                                const double2* __restrict__ Pm,
-                                                                const double2* __restrict__ M1,
-                                                                const double2* __restrict__ M2,
-                                                                const double2* __restrict__ Xm,
-                                                                const double2* __restrict__ D2, int n,
-                                                                long long G, double2* __restrict__ out) {
-  extern __shared__ double2 rsm[];
-  double2* sm = rsm;               // n*n: M1 + M2
-  double2* sd = sm + n * n;        // n*n: D2
-  double2* sp = sd + n * n;        // n x TXO
-  double2* sx = sp + n * TXO;      // n x TXO
-  const int lx = threadIdx.x, ty = threadIdx.y, tid = ty * TXO + lx;
-  for (int e = tid; e < n * n; e += TXO * blockDim.y) {
-    sm[e] = cadd(M1[e], M2[e]);
-    sd[e] = D2[e];
-  }
-  const long long x = blockIdx.x * (long long)TXO + lx;
-  const bool ok = x < G;
-  for (int j = ty; j < n; j += blockDim.y) {
-    sp[j * TXO + lx] = ok ? Pm[(long long)j * G + x] : make_double2(0.0, 0.0);
-    sx[j * TXO + lx] = ok ? Xm[(long long)j * G + x] : make_double2(0.0, 0.0);
-  }
-  __syncthreads();
-  if (!ok) return;
-  for (int i = ty; i < n; i += blockDim.y) {
-    double2 a = make_double2(0.0, 0.0);
-    for (int j = 0; j < n; ++j) {
-      cfma(a, sp[j * TXO + lx], sm[j + n * i]);
-      cfma(a, sx[j * TXO + lx], sd[j + n * i]);
-    }
-    out[(long long)i * G + x] = csub(Tm[(long long)i * G + x], a);
-  }
+// a += b (n^2 elements)
+__global__ void mat_add_kernel(double2* __restrict__ a, const double2* __restrict__ b, int nn) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e < nn) a[e] = cadd(a[e], b[e]);
 }
 
 // acc = a * acc + b * in  (or acc = b * in when `first`)
@@ -369,9 +485,7 @@ namespace {
 // the kernels' shared-memory limit: one fixed value (race-free across threads)
 int rhs_attrs() {
   static const cudaError_t attr = [] {
-    for (const void* k : {(const void*)mix_kernel, (const void*)redpot_kernel, (const void*)dots_kernel<DCH>,
-                          (const void*)dots_kernel<4 * DCH>,
-                          (const void*)project_kernel, (const void*)jac_combine_kernel,
+    for (const void* k : {(const void*)redpot_kernel, (const void*)dots_kernel<DCH>, (const void*)dots_kernel<4 * DCH>,
                           (const void*)blend2_kernel, (const void*)blendq_build_kernel,
                           (const void*)blendq_apply_kernel}) {
       const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kRhsSmemMax);
@@ -383,56 +497,111 @@ int rhs_attrs() {
   return SINCGPU_OK;
 }
 
+template <int NS, int NT>
+int launch_lin_t(Ctx& c, const double2* base, const double2* s0, const double2* m0, const double2* s1,
+                 const double2* m1, double sgn, double2* out) {
+  constexpr size_t sm = sizeof(double) * NS * 2 * NT * NT * 32;
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(lin_kernel<NS, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  SG_CUDA(attr);
+  lin_kernel<NS, NT><<<ceil_div(c.G, 8 * LMT * kLinWarps), 32 * kLinWarps, sm, c.stream>>>(base, s0, m0, s1, m1, sgn,
+                                                                                          c.nspf, c.G, out);
+  SG_LAUNCHED();
+  return SINCGPU_OK;
+}
+
+// out = [base] + sgn (s0 m0 [+ s1 m1]) over the orbitals (lin_kernel)
+int launch_lin(Ctx& c, const double2* base, const double2* s0, const double2* m0, const double2* s1,
+               const double2* m1, double sgn, double2* out) {
+#define SG_LIN(NT)                                                                                \
+  case NT:                                                                                        \
+    return s1 ? launch_lin_t<2, NT>(c, base, s0, m0, s1, m1, sgn, out)                            \
+              : launch_lin_t<1, NT>(c, base, s0, m0, nullptr, nullptr, sgn, out);
+  switch ((c.nspf + 3) / 4) {
+    SG_LIN(1)
+    SG_LIN(2)
+    SG_LIN(3)
+    SG_LIN(4)
+    SG_LIN(5)
+    SG_LIN(6)
+    SG_LIN(7)
+    default:
+      SG_LIN(8)
+  }
+#undef SG_LIN
+}
+
+template <int NT>
+int launch_dots_mma(Ctx& c, const double2* P, const double2* T, const double2* X, const double2* O, double2* D,
+                    double2* part) {
+  constexpr size_t sm = sizeof(double) * kDotWarps * NT * NT * 64;
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(dots_mma_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  SG_CUDA(attr);
+  const int nb = (int)std::min<long long>(kDotBlocks, ceil_div(c.G, dot_points(NT)));
+  dots_mma_kernel<NT><<<nb, 32 * kDotWarps, sm, c.stream>>>(P, T, X, O, c.nspf, c.G, part, D, c.d_count);
+  SG_LAUNCHED();
+  return SINCGPU_OK;
+}
+
 // one warp per orbital (n <= 32): every warp of a block has the same share of
 // the per-orbital loops
 dim3 tile_for(int n) { return dim3(TXO, (unsigned)std::max(1, std::min(n, kMaxOrbRhs))); }
 
-size_t smem_mix(int n) { return sizeof(double2) * ((size_t)n * n + (size_t)n * TXO); }
 size_t smem_redpot(int n) { return sizeof(double2) * ((size_t)n * n + 2 * (size_t)n * TXO); }
 size_t smem_dots(int n, int bl = DCH) { return sizeof(double2) * (size_t)n * bl; }
-size_t smem_jac(int n) { return sizeof(double2) * (2 * (size_t)n * n + 2 * (size_t)n * TXO); }
 
-int launch_dots(Ctx& c, const double2* P, const double2* T, double2* D, double2* part, bool wide = false) {
+// D = <P|T> [+ <X|O>]: the tensor-core form up to 16 orbitals (its accumulators: 128
+// registers a thread at 16), beyond that one pass of dots_kernel per pair
+int launch_dots(Ctx& c, const double2* P, const double2* T, const double2* X, const double2* O, double2* D,
+                double2* part) {
   const int n = c.nspf;
-  wide = wide && smem_dots(n, 4 * DCH) <= (size_t)kRhsSmemMax;
+  switch ((n + 3) / 4) {
+    case 1: return launch_dots_mma<1>(c, P, T, X, O, D, part);
+    case 2: return launch_dots_mma<2>(c, P, T, X, O, D, part);
+    case 3: return launch_dots_mma<3>(c, P, T, X, O, D, part);
+    case 4: return launch_dots_mma<4>(c, P, T, X, O, D, part);
+    default: break;
+  }
+  const bool wide = smem_dots(n, 4 * DCH) <= (size_t)kRhsSmemMax;
   const int nb = ceil_div(c.G, wide ? 4 * DCH : DCH);
-  if (wide)
-    dots_kernel<4 * DCH><<<nb, tile_for(n), smem_dots(n, 4 * DCH), c.stream>>>(P, T, n, c.G, part);
-  else
-    dots_kernel<DCH><<<nb, tile_for(n), smem_dots(n), c.stream>>>(P, T, n, c.G, part);
-  SG_LAUNCHED();
-  dots_reduce_kernel<<<n * n, 128, 0, c.stream>>>(part, nb, n * n, D);
-  SG_LAUNCHED();
+  double2* second = part + (size_t)orbital_dots_scratch(c) * n * n - (size_t)n * n;  // the scratch's last n^2
+  for (int s = 0; s < (X ? 2 : 1); ++s) {
+    if (wide)
+      dots_kernel<4 * DCH><<<nb, tile_for(n), smem_dots(n, 4 * DCH), c.stream>>>(s ? X : P, s ? O : T, n, c.G, part);
+    else
+      dots_kernel<DCH><<<nb, tile_for(n), smem_dots(n), c.stream>>>(s ? X : P, s ? O : T, n, c.G, part);
+    SG_LAUNCHED();
+    dots_reduce_kernel<<<n * n, 128, 0, c.stream>>>(part, nb, n * n, s ? second : D);
+    SG_LAUNCHED();
+  }
+  if (X) {
+    mat_add_kernel<<<ceil_div(n * n, 256), 256, 0, c.stream>>>(D, second, n * n);
+    SG_LAUNCHED();
+  }
   return SINCGPU_OK;
 }
 
 }  // namespace
 
-int orbital_dots_scratch(const Ctx& c) { return ceil_div(c.G, DCH); }
+int orbital_dots_scratch(const Ctx& c) { return std::max(ceil_div(c.G, DCH), kDotBlocks) + 1; }
 
-int orbital_dots(Ctx& c, const double2* P, const double2* T, double2* D, double2* part) {
+int orbital_dots(Ctx& c, const double2* P, const double2* T, double2* D, double2* part, const double2* X,
+                 const double2* O) {
   SG_CHECK(c.nspf <= kMaxOrbRhs, SINCGPU_ERANGE, "at most %d orbitals", kMaxOrbRhs);
   SG_TRY(rhs_attrs());
-  return launch_dots(c, P, T, D, part, true);
+  return launch_dots(c, P, T, X, O, D, part);
 }
 
 int orbital_mix(Ctx& c, const double2* in, const double2* mat, double2* out) {
-  const int n = c.nspf;
-  SG_CHECK(n <= kMaxOrbRhs, SINCGPU_ERANGE, "at most %d orbitals", kMaxOrbRhs);
-  SG_TRY(rhs_attrs());
-  mix_kernel<<<ceil_div(c.G, TXO), tile_for(n), smem_mix(n), c.stream>>>(in, mat, n, c.G, out);
-  SG_LAUNCHED();
-  return SINCGPU_OK;
+  SG_CHECK(c.nspf <= kMaxOrbRhs, SINCGPU_ERANGE, "at most %d orbitals", kMaxOrbRhs);
+  return launch_lin(c, nullptr, in, mat, nullptr, nullptr, 1.0, out);
 }
 
-int jac_combine(Ctx& c, const double2* T, const double2* P, const double2* M1, const double2* M2,
-                const double2* X, const double2* D2, double2* out) {
-  const int n = c.nspf;
-  SG_CHECK(n <= kMaxOrbRhs, SINCGPU_ERANGE, "at most %d orbitals", kMaxOrbRhs);
-  SG_TRY(rhs_attrs());
-  jac_combine_kernel<<<ceil_div(c.G, TXO), tile_for(n), smem_jac(n), c.stream>>>(T, P, M1, M2, X, D2, n, c.G, out);
-  SG_LAUNCHED();
-  return SINCGPU_OK;
+int jac_combine(Ctx& c, const double2* T, const double2* P, const double2* M, const double2* X, const double2* D2,
+                double2* out) {
+  SG_CHECK(c.nspf <= kMaxOrbRhs, SINCGPU_ERANGE, "at most %d orbitals", kMaxOrbRhs);
+  return launch_lin(c, T, P, M, X, D2, -1.0, out);
 }
 
 int axpby(Ctx& c, double2* acc, const double2* in, double a, double b, long long len, bool first) {
@@ -468,7 +637,7 @@ int rhs_temps(Ctx& c, RhsTemps& t) {
   SG_CHECK(n <= kMaxOrbRhs, SINCGPU_ERANGE, "at most %d orbitals", kMaxOrbRhs);
   SG_TRY(rhs_attrs());
   const long long G = c.G;
-  const int nb = ceil_div(G, DCH);
+  const int nb = orbital_dots_scratch(c);
   const size_t need = sizeof(double2) * (3 * (size_t)n * G + (size_t)nb * n * n + (size_t)n * n);
   SG_TRY(c.ws_rhs.ensure(need));
   t.Y = (double2*)c.ws_rhs.ptr;
@@ -493,8 +662,7 @@ int actreduced_pre(Ctx& c, const double2* phi, const double2* denmat, double zfi
   const int n = c.nspf;
   {
     ProfScope ps(c, ST_RHS_MIX);
-    mix_kernel<<<ceil_div(c.G, TXO), tile_for(n), smem_mix(n), c.stream>>>(phi, denmat, n, c.G, t.Y);
-    SG_LAUNCHED();
+    SG_TRY(orbital_mix(c, phi, denmat, t.Y));
   }
   return mult_ke(c, t.Y, t.S, n, true, zfield);
 }
@@ -508,11 +676,8 @@ int actreduced_ke(Ctx& c, const double2* phi, double zfield) {
 int actreduced_mix_ke(Ctx& c, const double2* denmat) {
   RhsTemps t;
   SG_TRY(rhs_temps(c, t));
-  const int n = c.nspf;
   ProfScope ps(c, ST_RHS_MIX);
-  mix_kernel<<<ceil_div(c.G, TXO), tile_for(n), smem_mix(n), c.stream>>>(t.Y, denmat, n, c.G, t.S);
-  SG_LAUNCHED();
-  return SINCGPU_OK;
+  return orbital_mix(c, t.Y, denmat, t.S);
 }
 
 bool actreduced_blend2_fits(int n) {
@@ -574,18 +739,17 @@ int actreduced_blendq(Ctx& c, const double2* x, double2 timefac, double zfield, 
   return SINCGPU_OK;
 }
 
-int actreduced_temps(Ctx& c, double2** S, double2** T, double2** part) {
+int actreduced_temps(Ctx& c, double2** S, double2** T) {
   RhsTemps t;
   SG_TRY(rhs_temps(c, t));
   *S = t.S;
   *T = t.T;
-  if (part) *part = t.part;
   return SINCGPU_OK;
 }
 
 int actreduced_post(Ctx& c, const double2* phi, const double2* proj, const double2* invdenmat,
                     const double2* redpot, double2 timefac, int dentimeflag, int projflag, double2* out,
-                    bool t_ready, bool dots_ready) {
+                    bool t_ready) {
   RhsTemps t;
   SG_TRY(rhs_temps(c, t));
   const int n = c.nspf;
@@ -601,17 +765,8 @@ int actreduced_post(Ctx& c, const double2* phi, const double2* proj, const doubl
   }
   if (projflag == 1) {
     ProfScope ps(c, ST_RHS_PROJ);
-    if (dots_ready) {
-      dots_reduce_kernel<<<n * n, 128, 0, c.stream>>>(part, ceil_div(G, DCH), n * n, D);
-      SG_LAUNCHED();
-    } else {
-      // above 10 orbitals no GEMM epilogue forms 64-point partials, so the dots
-      // take 256-point blocks (a quarter of the partials; 81^3, 16 orbitals: the
-      // 64-point form took 0.27 ms)
-      SG_TRY(launch_dots(c, proj, T, D, part, n > 10));
-    }
-    project_kernel<<<bt, tile_for(n), smem_mix(n), c.stream>>>(T, proj, D, n, G, out);
-    SG_LAUNCHED();
+    SG_TRY(launch_dots(c, proj, T, nullptr, nullptr, D, part));
+    SG_TRY(launch_lin(c, T, proj, D, nullptr, nullptr, -1.0, out));
   }
   return SINCGPU_OK;
 }
