@@ -76,7 +76,7 @@ struct IntCache {
   int* dev = nullptr;
   size_t cap = 0;
 };
-enum IntSlot { IC_PA = 0, IC_PB, IC_LUT, IC_TMAP, IC_COUNT };
+enum IntSlot { IC_PA = 0, IC_PB, IC_LUT, IC_TMAP, IC_TROWS, IC_ROWOF, IC_RROWS, IC_TMAP_PACKED, IC_COUNT };
 
 // saved variables of the orbital exponential propagator (expospfprop)
 struct OrbPropState {

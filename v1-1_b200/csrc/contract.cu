@@ -14,6 +14,8 @@
 //   reducedpot: out = sum_p r_p A_p + s_p B_p with A_p = G(c,d)+G(d,c),
 //       B_p = i(G(c,d)-G(d,c)) for c<d and A_p = G(c,c), B_p = iG(c,c) for c=d,
 //   i.e. [r|s] (G x 2U) times a real 2U x 2n^2 matrix.
+// The n diagonal pairs (c = d) are real, so in FP64 their imaginary rows (zero up to
+// rounding) are left out and 2U = n(n+1) becomes n^2 in both (hermitian_rows).
 // Compared with the complex contractions of the reference this is 4x (twoematel)
 // and 2x (reducedpot) fewer flops.  Without the symmetry (phi1 != phi2) all n^2
 // ordered pairs are used with the plain complex identities.
@@ -237,8 +239,9 @@ template <int R, bool SYM, int KT>
 __global__ void __launch_bounds__(64 * R, 1) twoe_dmma_kernel(const double2* __restrict__ phi1,
                                                               const double2* __restrict__ phi2,
                                                               const int* __restrict__ pa, const int* __restrict__ pb,
-                                                              const double* __restrict__ Rpl, int npair, int nspf,
-                                                              long long G, int ntn, long long xper,
+                                                              const double* __restrict__ Rpl,
+                                                              const int* __restrict__ rows, int M, int npair,
+                                                              int nspf, long long G, int ntn, long long xper,
                                                               double* __restrict__ part, int strict) {
   constexpr int TT = 16 * R;
   constexpr int TS = KT + 4;  // shared-memory row stride (doubles), 4 mod 16
@@ -251,7 +254,7 @@ __global__ void __launch_bounds__(64 * R, 1) twoe_dmma_kernel(const double2* __r
   int* sa = reinterpret_cast<int*>(fsm + 6 * nspf * KT);
   int* sb = sa + TT;
   int* sc = sb + TT;
-  const int M = 2 * npair;
+  __shared__ int srow[TT];  // the tile's columns' rows of Rpl, -1 beyond M
   // tile (tm, tn): SYM CTAs take the diagonal tiles (blockIdx.x = tm = tn); the
   // others the upper-triangle tiles, the diagonal included unless `strict`
   int tm = 0, tn = 0;
@@ -271,11 +274,12 @@ __global__ void __launch_bounds__(64 * R, 1) twoe_dmma_kernel(const double2* __r
   const int tid = threadIdx.x;
   for (int i = tid; i < TT; i += NTH) {
     const int m = m0 + i;
+    srow[i] = n0 + i < M ? (rows ? rows[n0 + i] : n0 + i) : -1;
     if (m < M) {
-      const int p = m % npair;
+      const int r = rows ? rows[m] : m, p = r % npair;
       sa[i] = pa[p];
       sb[i] = pb[p];
-      sc[i] = m / npair;
+      sc[i] = r / npair;
     } else {
       sa[i] = 0;
       sb[i] = 0;
@@ -298,10 +302,10 @@ __global__ void __launch_bounds__(64 * R, 1) twoe_dmma_kernel(const double2* __r
     double* b = Bs + st * TT * TS;
     for (int i = tid; i < KT * TT; i += NTH) {
       const int nn = i / KT, k = i % KT;
-      const int n = n0 + nn;
+      const int r = srow[nn];
       const long long x = x0 + k;
-      const bool ok = n < M && x < xe;
-      cp_async8(&b[nn * TS + k], ok ? (const void*)(Rpl + (long long)n * G + x) : (const void*)Rpl, ok);
+      const bool ok = r >= 0 && x < xe;
+      cp_async8(&b[nn * TS + k], ok ? (const void*)(Rpl + (long long)r * G + x) : (const void*)Rpl, ok);
     }
     cp_async_commit();
   };
@@ -410,6 +414,137 @@ __global__ void __launch_bounds__(64 * R, 1) twoe_dmma_kernel(const double2* __r
   }
 }
 
+// twoematel GEMM of hermitian pairs with more rows than one tile of twoe_dmma_kernel
+// holds (13 to 16 orbitals), FP64 tensor cores.  C = A^T B is
+// symmetric, so the M x M outputs are cut into 32 x 32 patches and only the NP (NP + 1) / 2
+// patches on and above the diagonal are formed, one per warp (4 x 4 fragments, 8 fragment
+// loads for 16 MMAs); gridDim.x CTAs of the same K range share the patches, each staging
+// all rows: the pair products of the next 16 points are formed between the MMAs of the
+// current ones (both parts of a pair at once), the potentials arrive by cp.async a stage
+// ahead, one barrier per stage.
+// What bounds it: the FP64 tensor pipe, G M (M + 32) flops (81^3, 16 orbitals: 1.06 ms at
+// 37 TF/s).  Measured there 2.92 ms (three 144 x 144 tiles, all their fragments) -> 2.23.
+constexpr int PK = 16, PTS = PK + 4, kPatch = 32, kPatchOrb = 16;
+constexpr int kPatchRows = kPatchOrb * kPatchOrb, kPatchPairs = kPatchOrb * (kPatchOrb + 1) / 2;
+__global__ void __launch_bounds__(512, 1) twoe_patch_kernel(const double2* __restrict__ phi,
+                                                            const int* __restrict__ pa, const int* __restrict__ pb,
+                                                            const double* __restrict__ Rpl,
+                                                            const int* __restrict__ rows,
+                                                            const int* __restrict__ rowof, int M, int npair, int nspf,
+                                                            long long G, long long xper, double* __restrict__ part) {
+  extern __shared__ __align__(16) double dsm[];
+  const int NP = (M + kPatch - 1) / kPatch, MP = NP * kPatch;
+  double* As = dsm;                                              // [2][MP][PTS]
+  double* Bs = As + 2 * MP * PTS;                                // [2][MP][PTS]
+  double2* fsm = reinterpret_cast<double2*>(Bs + 2 * MP * PTS);  // [2][nspf][PK]
+  __shared__ int srow[kPatchRows];                 // rows of Rpl
+  __shared__ short4 spair[kPatchPairs];            // pair -> (a, b, row of Re, row of Im or -1)
+  const int tid = threadIdx.x, NTH = blockDim.x, warp = tid >> 5;
+  for (int i = tid; i < MP; i += NTH) srow[i] = i < M ? (rows ? rows[i] : i) : -1;
+  for (int i = tid; i < npair; i += NTH)
+    spair[i] = make_short4((short)pa[i], (short)pb[i], (short)(rowof ? rowof[i] : i),
+                           (short)(rowof ? rowof[npair + i] : npair + i));
+  for (int i = tid; i < 2 * MP * PTS; i += NTH) As[i] = 0.0;  // rows beyond M
+  // this warp's patch (pi <= pj)
+  int pi = 0, pj = blockIdx.x * (NTH >> 5) + warp;
+  const bool work = pj < NP * (NP + 1) / 2;
+  while (work && pj >= NP - pi) {
+    pj -= NP - pi;
+    ++pi;
+  }
+  pj += pi;
+  const long long xb = blockIdx.y * xper, xe = min(G, xb + xper);
+  const int nk = (int)((xe - xb + PK - 1) / PK);
+  auto load_raw = [&](int st, long long x0) {
+    for (int i = tid; i < nspf * PK; i += NTH) {
+      const int o = i / PK, k = i % PK;
+      const bool ok = x0 + k < xe;
+      cp_async16(fsm + (st * nspf + o) * PK + k, ok ? phi + (long long)o * G + x0 + k : phi, ok);
+    }
+  };
+  auto load_b = [&](int st, long long x0) {
+    for (int i = tid; i < MP * PK; i += NTH) {
+      const int r = srow[i / PK], k = i % PK;
+      const bool ok = r >= 0 && x0 + k < xe;
+      cp_async8(Bs + (st * MP + i / PK) * PTS + k, ok ? Rpl + (long long)r * G + x0 + k : Rpl, ok);
+    }
+  };
+  const int items = npair * PK, per = (items + 4 * NTH - 1) / (4 * NTH);  // products per thread and K = 4 step
+  auto products = [&](int st, int ab, int q) {
+    const double2* f = fsm + st * nspf * PK;
+    double* A = As + ab * MP * PTS;
+    for (int u = 0; u < per; ++u) {
+      const int i = tid + (q * per + u) * NTH;
+      if (i >= items) break;
+      const int k = i % PK;
+      const short4 p = spair[i / PK];
+      const double2 v = cmulc(f[p.x * PK + k], f[p.y * PK + k]);
+      A[p.z * PTS + k] = v.x;
+      if (p.w >= 0) A[p.w * PTS + k] = v.y;
+    }
+  };
+  double acc[4][4][2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  const int g8 = (tid & 31) >> 2, t4 = tid & 3;
+  __syncthreads();  // tables
+  if (nk > 0) {
+    load_raw(0, xb);
+    cp_async_commit();
+    load_b(0, xb);
+    if (nk > 1) load_raw(1, xb + PK);
+    cp_async_commit();
+    cp_async_wait<1>();
+    __syncthreads();
+    for (int q = 0; q < 4; ++q) products(0, 0, q);
+  }
+  for (int t = 0; t < nk; ++t) {
+    const int cur = t & 1;
+    cp_async_wait<0>();  // potentials of stage t, orbitals of stage t + 1
+    __syncthreads();     // products of stage t; stage t - 1 fully consumed
+    if (t + 1 < nk) load_b(cur ^ 1, xb + (long long)(t + 1) * PK);
+    if (t + 2 < nk) load_raw(cur, xb + (long long)(t + 2) * PK);
+    cp_async_commit();
+    const double* A = As + (cur * MP + pi * kPatch + g8) * PTS + t4;
+    const double* B = Bs + (cur * MP + pj * kPatch + g8) * PTS + t4;
+#pragma unroll
+    for (int k4 = 0; k4 < PK; k4 += 4) {
+      if (work) {
+        double a[4], b[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          a[i] = A[8 * i * PTS + k4];
+          b[i] = B[8 * i * PTS + k4];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) dmma_884(acc[i][j], a[i], b[j]);
+      }
+      if (t + 1 < nk) products(cur ^ 1, cur ^ 1, k4 / 4);
+    }
+  }
+  if (!work) return;
+  double* out = part + (long long)blockIdx.y * M * M;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int m = pi * kPatch + 8 * i + g8;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int n = pj * kPatch + 8 * j + 2 * t4;
+      if (m < M && n < M) out[(long long)m * M + n] = acc[i][j][0];
+      if (m < M && n + 1 < M) out[(long long)m * M + n + 1] = acc[i][j][1];
+    }
+  }
+}
+
+static size_t twoe_patch_smem(int M, int n) {
+  const int MP = ceil_div(M, kPatch) * kPatch;
+  return sizeof(double) * 4 * (size_t)MP * PTS + sizeof(double2) * 2 * (size_t)n * PK;
+}
+
 // C[m][n] = sum_s part[s][m][n] (deterministic): a CTA owns 32 consecutive
 // elements; its 8 warps sum interleaved eighths of the split range (warp g takes
 // splits g, g + 8, ...) in a fixed order and warp 0 adds the eight partial sums in
@@ -441,14 +576,15 @@ __global__ void __launch_bounds__(256) split_reduce_kernel(const double* __restr
 
 // twoematel(a1,b1,a2,b2) from C = [[UR,US],[VR,VS]]
 // lut[a + n*b] = 2*p + conj  (hermitian pairs a<=b), or p for the general list.
+// rowof[p], rowof[npair + p]: the rows of C with pair p's real and imaginary part (-1: zero)
 __global__ void twoe_assemble_kernel(const double* __restrict__ C, const int* __restrict__ lut,
-                                     int npair, int n, int herm, double2* __restrict__ out) {
+                                     const int* __restrict__ rowof, int M, int npair, int n, int herm,
+                                     double2* __restrict__ out) {
   long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long n4 = (long long)n * n * n * n;
   if (idx >= n4) return;
   int a1 = (int)(idx % n), b1 = (int)((idx / n) % n);
   int a2 = (int)((idx / ((long long)n * n)) % n), b2 = (int)(idx / ((long long)n * n * n));
-  const int M = 2 * npair;
   int lp = lut[a1 + n * b1], lq = lut[a2 + n * b2];
   int p, q, cp = 0, cq = 0;
   if (herm) {
@@ -460,8 +596,10 @@ __global__ void twoe_assemble_kernel(const double* __restrict__ C, const int* __
     p = lp;
     q = lq;
   }
-  double UR = C[(long long)p * M + q], US = C[(long long)p * M + npair + q];
-  double VR = C[(long long)(npair + p) * M + q], VS = C[(long long)(npair + p) * M + npair + q];
+  auto row = [&](int r) { return rowof ? rowof[r] : r; };
+  const int u = row(p), v = row(npair + p), rr = row(q), ss = row(npair + q);
+  auto at = [&](int i, int j) { return i >= 0 && j >= 0 ? C[(long long)i * M + j] : 0.0; };
+  const double UR = at(u, rr), US = at(u, ss), VR = at(v, rr), VS = at(v, ss);
   double2 r;
   if (!cp && !cq)
     r = make_double2(UR - VS, US + VR);
@@ -480,18 +618,18 @@ static size_t twoe_pipe_smem(int R, int KT, int n) {
   return sizeof(double) * 5 * (size_t)(16 * R) * (KT + 4) + sizeof(double2) * 6 * (size_t)n * KT +
          sizeof(int) * 3 * (size_t)(16 * R);
 }
-constexpr int kTwoeSmemMax = 227 * 1024;
+constexpr int kTwoeSmemMax = 226 * 1024;  // (the kernels' static tables beside it)
 
 template <int RR, bool SYM, int KT>
 static int launch_twoe_pipe_t(Ctx& c, dim3 grid, size_t bytes, const double2* phi1, const double2* phi2,
-                              const int* d_pa, const int* d_pb, const double* Rpl, int npair, int ntn,
-                              long long xper, double* part, int strict) {
+                              const int* d_pa, const int* d_pb, const double* Rpl, const int* d_rows, int M,
+                              int npair, int ntn, long long xper, double* part, int strict) {
   // process-wide attribute, one fixed value (thread-safe static initialisation)
   static const cudaError_t attr = cudaFuncSetAttribute(twoe_dmma_kernel<RR, SYM, KT>,
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, kTwoeSmemMax);
   SG_CUDA(attr);
-  twoe_dmma_kernel<RR, SYM, KT><<<grid, 64 * RR, bytes, c.stream>>>(phi1, phi2, d_pa, d_pb, Rpl, npair, c.nspf,
-                                                                     c.G, ntn, xper, part, strict);
+  twoe_dmma_kernel<RR, SYM, KT><<<grid, 64 * RR, bytes, c.stream>>>(phi1, phi2, d_pa, d_pb, Rpl, d_rows, M, npair,
+                                                                     c.nspf, c.G, ntn, xper, part, strict);
   return SINCGPU_OK;
 }
 
@@ -499,17 +637,17 @@ static int launch_twoe_pipe_t(Ctx& c, dim3 grid, size_t bytes, const double2* ph
 // barriers of 16-point stages; the same bits), else 16
 template <int RR>
 static int launch_twoe_pipe(Ctx& c, dim3 grid, bool sym, const double2* phi1, const double2* phi2,
-                            const int* d_pa, const int* d_pb, const double* Rpl, int npair, int ntn,
-                            long long xper, double* part, int strict = 0) {
+                            const int* d_pa, const int* d_pb, const double* Rpl, const int* d_rows, int M,
+                            int npair, int ntn, long long xper, double* part, int strict = 0) {
   const size_t b32 = twoe_pipe_smem(RR, 32, c.nspf), b16 = twoe_pipe_smem(RR, 16, c.nspf);
   if (b32 <= (size_t)kTwoeSmemMax)
-    return sym ? launch_twoe_pipe_t<RR, true, 32>(c, grid, b32, phi1, phi2, d_pa, d_pb, Rpl, npair, ntn, xper, part,
+    return sym ? launch_twoe_pipe_t<RR, true, 32>(c, grid, b32, phi1, phi2, d_pa, d_pb, Rpl, d_rows, M, npair, ntn, xper, part,
                                                   0)
-               : launch_twoe_pipe_t<RR, false, 32>(c, grid, b32, phi1, phi2, d_pa, d_pb, Rpl, npair, ntn, xper,
+               : launch_twoe_pipe_t<RR, false, 32>(c, grid, b32, phi1, phi2, d_pa, d_pb, Rpl, d_rows, M, npair, ntn, xper,
                                                    part, strict);
-  return sym ? launch_twoe_pipe_t<RR, true, 16>(c, grid, b16, phi1, phi2, d_pa, d_pb, Rpl, npair, ntn, xper, part,
+  return sym ? launch_twoe_pipe_t<RR, true, 16>(c, grid, b16, phi1, phi2, d_pa, d_pb, Rpl, d_rows, M, npair, ntn, xper, part,
                                                 0)
-             : launch_twoe_pipe_t<RR, false, 16>(c, grid, b16, phi1, phi2, d_pa, d_pb, Rpl, npair, ntn, xper, part,
+             : launch_twoe_pipe_t<RR, false, 16>(c, grid, b16, phi1, phi2, d_pa, d_pb, Rpl, d_rows, M, npair, ntn, xper, part,
                                                  strict);
 }
 
@@ -525,20 +663,49 @@ static void pair_lut(int n, const int* pa, const int* pb, int npair, bool herm, 
   }
 }
 
+// Rows of the planar potentials [Re of the pairs | Im of the pairs] that the contractions
+// use for a hermitian pair list in FP64: all but the imaginary rows of the diagonal pairs
+// (n^2 of n (n + 1)), and for each planar row its place among them (-1: left out).
+static void hermitian_rows(const int* pa, const int* pb, int npair, std::vector<int>& rows, std::vector<int>& rowof) {
+  rows.clear();
+  rowof.assign(2 * (size_t)npair, -1);
+  for (int r = 0; r < 2 * npair; ++r) {
+    const int p = r % npair;
+    if (r >= npair && pa[p] == pb[p]) continue;
+    rowof[r] = (int)rows.size();
+    rows.push_back(r);
+  }
+}
+// whether they may: the potentials' diagonal imaginary parts are zero up to FP64 rounding
+// (FP32 potentials keep all rows: theirs are rounding of 1e-8)
+static bool drop_rows(const Ctx& c, bool herm) { return herm && !c.coul_fp32; }
+
 int twoe_matel(Ctx& c, const double2* phi1, const double2* phi2, const int* h_pa, const int* h_pb,
                int npair, const double* Rpl, bool herm, double2* twoematel) {
   const int n = c.nspf;
   SG_CHECK(n <= kMaxOrb, SINCGPU_ERANGE, "at most %d orbitals (got %d)", kMaxOrb, n);
-  const int M = 2 * npair;
+  // the pipelined kernels copy whole complex values (16 bytes)
+  const bool pipe = ((uintptr_t)phi1 % 16 == 0) && ((uintptr_t)phi2 % 16 == 0);
+  const bool drop = drop_rows(c, herm) && c.twoe_dmma && pipe;
+  std::vector<int> rows, rowof;
+  if (drop) hermitian_rows(h_pa, h_pb, npair, rows, rowof);
+  const int M = drop ? (int)rows.size() : 2 * npair;
   // register block R: the smallest of 2..9 whose 16R tile holds M, else 8 (multi-tile)
   // tile edge 16R with the least padding of M (ties: the larger tile)
   int R = 2;
   for (int r = 2; r <= 9; ++r)
     if (ceil_div(M, 16 * r) * 16 * r <= ceil_div(M, 16 * R) * 16 * R) R = r;
   if (c.twoe_tile >= 2 && c.twoe_tile <= 9) R = c.twoe_tile;
-  const int TT = 16 * R;
+  // hermitian pairs in more rows than one tile (13 to 16 orbitals): patches of the triangle
+  // (twoe_patch_kernel), up to the rows whose stages fit shared memory.  FP32 potentials
+  // keep the tiles: their pair matrix is symmetric to 1e-8 only, so which half is formed
+  // would show in the result.
+  const bool patch = drop && c.twoe_tile == 0 && !c.twoe_symdiag && M > 144 && n <= kPatchOrb;
+  const int npatch = ceil_div(M, kPatch) * (ceil_div(M, kPatch) + 1) / 2;
+  const int groups = patch ? ceil_div(npatch, 16) : 1;  // CTAs that share the patches of a K range
+  const int TT = patch ? kPatch : 16 * R;
   const int ntm = ceil_div(M, TT), ntn = ntm;
-  const int ntiles = ntm * (ntm + 1) / 2;  // upper triangle
+  const int ntiles = patch ? groups : ntm * (ntm + 1) / 2;  // upper triangle
   long long target = 148;  // one 256-thread CTA per SM (R x R accumulators per thread)
   int nsplit = (int)std::max(1LL, std::min((long long)ceil_div(c.G, TK), std::max(1LL, target / ntiles)));
   long long xper = ((c.G + nsplit - 1) / nsplit + TK - 1) / TK * TK;
@@ -548,21 +715,33 @@ int twoe_matel(Ctx& c, const double2* phi1, const double2* phi2, const int* h_pa
   SG_TRY(c.ws_twoe.ensure(need));
   double* part = (double*)c.ws_twoe.ptr;
   double* C = part + MM * nsplit;
-  const int *d_pa, *d_pb, *d_lut;
+  const int *d_pa, *d_pb, *d_lut, *d_rows = nullptr, *d_rowof = nullptr;
   std::vector<int> lut;
   pair_lut(n, h_pa, h_pb, npair, herm, lut);
   SG_TRY(cached_ints(c, IC_PA, h_pa, npair, &d_pa));
   SG_TRY(cached_ints(c, IC_PB, h_pb, npair, &d_pb));
   SG_TRY(cached_ints(c, IC_LUT, lut.data(), (size_t)n * n, &d_lut));
+  if (drop) {
+    SG_TRY(cached_ints(c, IC_TROWS, rows.data(), rows.size(), &d_rows));
+    SG_TRY(cached_ints(c, IC_ROWOF, rowof.data(), rowof.size(), &d_rowof));
+  }
   bool sym = false;
-  {
+  if (patch) {
+    ProfScope ps(c, ST_TWOE_GEMM);
+    static const cudaError_t attr =
+        cudaFuncSetAttribute(twoe_patch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)twoe_patch_smem(kPatchRows, kPatchOrb));
+    SG_CUDA(attr);
+    const size_t bytes = twoe_patch_smem(M, n);
+    twoe_patch_kernel<<<dim3(groups, nsplit), 32 * ceil_div(npatch, groups), bytes, c.stream>>>(
+        phi1, d_pa, d_pb, Rpl, d_rows, d_rowof, M, npair, n, c.G, xper, part);
+    SG_LAUNCHED();
+  } else {
     ProfScope ps(c, ST_TWOE_GEMM);
     const int TS = c.twoe_dmma ? TK + 4 : TK + 1;
     const size_t sbytes = sizeof(double) * 3 * (size_t)TT * TS + sizeof(double2) * 4 * (size_t)n * TK +
                           sizeof(int) * 3 * (size_t)TT;
     const dim3 grid(ntiles, nsplit);
-    // the pipelined kernel copies whole complex values (16 bytes)
-    const bool pipe = ((uintptr_t)phi1 % 16 == 0) && ((uintptr_t)phi2 % 16 == 0);
     // hermitian pairs make the pair matrix symmetric: a diagonal tile needs only
     // its blocks on and below the diagonal (the SYM kernel); with several tiles
     // (option twoe_symdiag) the diagonal tiles take that kernel and the strictly
@@ -570,12 +749,12 @@ int twoe_matel(Ctx& c, const double2* phi1, const double2* phi2, const int* h_pa
     sym = pipe && herm && c.twoe_dmma && (ntm == 1 || c.twoe_symdiag);
 #define SG_TWOE_LAUNCH(RR, DM)                                                                             \
   if (DM && pipe && sym && ntm > 1) {                                                                      \
-    SG_TRY(launch_twoe_pipe<RR>(c, dim3(ntm, nsplit), true, phi1, phi2, d_pa, d_pb, Rpl, npair, ntn, xper,  \
-                                part));                                                                    \
+    SG_TRY(launch_twoe_pipe<RR>(c, dim3(ntm, nsplit), true, phi1, phi2, d_pa, d_pb, Rpl, d_rows, M, npair,  \
+                                ntn, xper, part));                                                         \
     SG_TRY(launch_twoe_pipe<RR>(c, dim3(ntm * (ntm - 1) / 2, nsplit), false, phi1, phi2, d_pa, d_pb, Rpl,   \
-                                npair, ntn, xper, part, 1));                                               \
+                                d_rows, M, npair, ntn, xper, part, 1));                                               \
   } else if (DM && pipe) {                                                                                 \
-    SG_TRY(launch_twoe_pipe<RR>(c, grid, sym, phi1, phi2, d_pa, d_pb, Rpl, npair, ntn, xper, part));        \
+    SG_TRY(launch_twoe_pipe<RR>(c, grid, sym, phi1, phi2, d_pa, d_pb, Rpl, d_rows, M, npair, ntn, xper, part));        \
   } else {                                                                                                 \
     static const cudaError_t attr = cudaFuncSetAttribute(                                                  \
         twoe_gemm3_kernel<RR, DM>, cudaFuncAttributeMaxDynamicSharedMemorySize,                            \
@@ -612,7 +791,7 @@ int twoe_matel(Ctx& c, const double2* phi1, const double2* phi2, const int* h_pa
   split_reduce_kernel<<<ceil_div(MM, 32), 256, 0, c.stream>>>(part, nsplit, M, TT, C);
   SG_LAUNCHED();
   const long long n4 = (long long)n * n * n * n;
-  twoe_assemble_kernel<<<ceil_div(n4, 256), 256, 0, c.stream>>>(C, d_lut, npair, n, herm ? 1 : 0,
+  twoe_assemble_kernel<<<ceil_div(n4, 256), 256, 0, c.stream>>>(C, d_lut, d_rowof, M, npair, n, herm ? 1 : 0,
                                                                  twoematel);
   SG_LAUNCHED();
   return SINCGPU_OK;
@@ -648,20 +827,36 @@ __global__ void build_w_kernel(const double2* __restrict__ tally, const int* __r
   Wm[idx] = (col & 1) ? v.y : v.x;
 }
 
-// Half-column W: columns c = 2t + {re, im} for the orbital pairs t = (kk, ii),
-// kk <= ii, listed in tmap (kk, ii interleaved).  With a hermitian pair list and a
-// 2-RDM of one A-vector (Gamma(c,d,k,i) = conj Gamma(d,c,i,k)), reducedpot(x,i,k)
-// = conj reducedpot(x,k,i), so these columns determine all of it.
+// Half-column W: columns c = 2t + {re, im} for the orbital pairs t = (kk, ii), kk <= ii,
+// listed in tmap (kk, ii interleaved).  With a hermitian pair list and a 2-RDM of one
+// A-vector (Gamma(c,d,k,i) = conj Gamma(d,c,i,k)), reducedpot(x,i,k) = conj
+// reducedpot(x,k,i), so these columns determine all of it.  In the packed form (rows
+// without the diagonal pairs' zeros) the diagonals reducedpot(x,k,k), which are real, share
+// column pairs at the end: an entry (-1 - k, k') stands for the real parts of k and k' (k'
+// = -1: none), and n (n + 1) columns become n^2.  rows: the potentials' rows (null: all).
 __global__ void build_w_half_kernel(const double2* __restrict__ tally, const int* __restrict__ pa,
-                                    const int* __restrict__ pb, const int* __restrict__ tmap, int npair, int n,
-                                    int nt, double* __restrict__ Wm) {
+                                    const int* __restrict__ pb, const int* __restrict__ tmap,
+                                    const int* __restrict__ rows, int K, int npair, int n, int nt,
+                                    double* __restrict__ Wm) {
   const int NC = 2 * nt;
   long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (idx >= 2LL * npair * NC) return;
+  if (idx >= (long long)K * NC) return;
   int k = (int)(idx / NC), col = (int)(idx % NC);
-  int p = k % npair, comp = k / npair;
+  const int r = rows ? rows[k] : k;
+  int p = r % npair, comp = r / npair;
   int cc = pa[p], d = pb[p];
-  const int t = col / 2, kk = tmap[2 * t], ii = tmap[2 * t + 1];
+  const int t = col / 2;
+  int kk = tmap[2 * t], ii = tmap[2 * t + 1];
+  bool im = col & 1;
+  if (kk < 0) {  // two diagonals
+    kk = im ? ii : -1 - kk;
+    ii = kk;
+    im = false;
+    if (kk < 0) {
+      Wm[idx] = 0.0;
+      return;
+    }
+  }
   long long tail = (long long)n * n * (kk + (long long)n * ii);
   double2 g1 = tally[cc + n * d + tail];
   double2 A, B;
@@ -675,7 +870,7 @@ __global__ void build_w_half_kernel(const double2* __restrict__ tally, const int
     B = make_double2(-g1.y, g1.x);
   }
   double2 v = comp == 0 ? A : B;
-  Wm[idx] = (col & 1) ? v.y : v.x;
+  Wm[idx] = im ? v.y : v.x;
 }
 
 constexpr int RM = 128, RK = 16;
@@ -779,8 +974,8 @@ constexpr int DAS = DM + 4;
 template <int FN>
 __device__ __forceinline__ void rp_dmma_mainloop(double (*As)[DK][DAS], double (*Bs)[DK][16 * FN + 4],
                                                  const double* __restrict__ Rpl, const double* __restrict__ Wm,
-                                                 int K, int NC, long long G, long long x0, int c0,
-                                                 double (&acc)[2][FN][2]) {
+                                                 const int* __restrict__ rows, int K, int NC, long long G,
+                                                 long long x0, int c0, double (&acc)[2][FN][2]) {
   constexpr int DN = 16 * FN;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
@@ -794,7 +989,8 @@ __device__ __forceinline__ void rp_dmma_mainloop(double (*As)[DK][DAS], double (
       const int k = i / DM, xx = i % DM;
       const long long x = x0 + xx;
       const bool ok = (k0 + k < K) && x < G;
-      cp_async8(&As[st][k][xx], ok ? (const void*)(Rpl + (long long)(k0 + k) * G + x) : (const void*)Rpl, ok);
+      const int r = ok && rows ? rows[k0 + k] : k0 + k;
+      cp_async8(&As[st][k][xx], ok ? (const void*)(Rpl + (long long)r * G + x) : (const void*)Rpl, ok);
     }
     for (int i = tid; i < DK * DN / 2; i += 256) {
       const int k = i / (DN / 2), cc = 2 * (i % (DN / 2));
@@ -816,6 +1012,7 @@ __device__ __forceinline__ void rp_dmma_mainloop(double (*As)[DK][DAS], double (
     if (kc + 1 < nk) load((kc + 1) % DST, (kc + 1) * DK);
 #pragma unroll
     for (int k4 = 0; k4 < DK; k4 += 4) {
+      if (kc * DK + k4 >= K) break;
       double a[2], b[FN];
 #pragma unroll
       for (int i = 0; i < 2; ++i) a[i] = As[st][k4 + t][wm + 8 * i + g];
@@ -849,6 +1046,11 @@ __device__ __forceinline__ void rp_dmma_store(const double (&acc)[2][FN][2], lon
       const double2 v = make_double2(acc[i][j][0], acc[i][j][1]);
       if (HALF) {
         const int tt = col / 2, kk = tmap[2 * tt], ii = tmap[2 * tt + 1];
+        if (kk < 0) {  // two real diagonals
+          out[(long long)(-1 - kk) * (n + 1) * G + x] = make_double2(v.x, 0.0);
+          if (ii >= 0) out[(long long)ii * (n + 1) * G + x] = make_double2(v.y, 0.0);
+          continue;
+        }
         out[(long long)(kk + n * ii) * G + x] = v;
         if (kk != ii) out[(long long)(ii + n * kk) * G + x] = make_double2(v.x, -v.y);
       } else {
@@ -858,16 +1060,22 @@ __device__ __forceinline__ void rp_dmma_store(const double (&acc)[2][FN][2], lon
   }
 }
 
+template <int FN>
+constexpr size_t rp_stage_bytes() { return sizeof(double) * DST * DK * ((size_t)DAS + 16 * FN + 4); }
+
 template <bool HALF, int FN>
-__global__ void __launch_bounds__(256, 3) rp_dmma_kernel(const double* __restrict__ Rpl, const double* __restrict__ Wm,
-                                                      int K, int NC, long long G, double2* __restrict__ out,
-                                                      const int* __restrict__ tmap, int n) {
-  __shared__ __align__(16) double As[DST][DK][DAS];
-  __shared__ __align__(16) double Bs[DST][DK][16 * FN + 4];
+__global__ void __launch_bounds__(256, FN <= 7 ? 3 : 2) rp_dmma_kernel(const double* __restrict__ Rpl,
+                                                                   const double* __restrict__ Wm,
+                                                                   const int* __restrict__ rows, int K, int NC,
+                                                                   long long G, double2* __restrict__ out,
+                                                                   const int* __restrict__ tmap, int n) {
+  extern __shared__ __align__(16) double rp_sm[];
+  auto As = reinterpret_cast<double (*)[DK][DAS]>(rp_sm);
+  auto Bs = reinterpret_cast<double (*)[DK][16 * FN + 4]>(rp_sm + DST * DK * DAS);
   const long long x0 = (long long)blockIdx.x * DM;
   const int c0 = blockIdx.y * 16 * FN;
   double acc[2][FN][2];
-  rp_dmma_mainloop<FN>(As, Bs, Rpl, Wm, K, NC, G, x0, c0, acc);
+  rp_dmma_mainloop<FN>(As, Bs, Rpl, Wm, rows, K, NC, G, x0, c0, acc);
   rp_dmma_store<HALF, FN>(acc, G, x0, c0, NC, tmap, n, out);
 }
 
@@ -882,7 +1090,8 @@ __global__ void __launch_bounds__(256, 3) rp_dmma_kernel(const double* __restric
 constexpr int RPV = DM + 2;  // tile row stride (doubles): conflict-free accumulator stores
 template <int FN>
 __global__ void __launch_bounds__(256, 3) rp_apply_kernel(const double* __restrict__ Rpl, const double* __restrict__ Wm,
-                                                       int K, int NC, long long G, double2* __restrict__ out,
+                                                       const int* __restrict__ rows, int packed, int K, int NC,
+                                                       long long G, double2* __restrict__ out,
                                                        const int* __restrict__ tmap, int n,
                                                        const double2* __restrict__ phi,
                                                        const double2* __restrict__ S,
@@ -893,7 +1102,7 @@ __global__ void __launch_bounds__(256, 3) rp_apply_kernel(const double* __restri
   auto Bs = reinterpret_cast<double (*)[DK][16 * FN + 4]>(rp_sm + DST * DK * DAS);
   const long long x0 = (long long)blockIdx.x * DM;
   double acc[2][FN][2];
-  rp_dmma_mainloop<FN>(As, Bs, Rpl, Wm, K, NC, G, x0, 0, acc);
+  rp_dmma_mainloop<FN>(As, Bs, Rpl, Wm, rows, K, NC, G, x0, 0, acc);
   rp_dmma_store<true, FN>(acc, G, x0, 0, NC, tmap, n, out);
   __syncthreads();  // every warp is done with the stages
   double* Vt = rp_sm;                                           // [NC][RPV]
@@ -932,8 +1141,17 @@ __global__ void __launch_bounds__(256, 3) rp_apply_kernel(const double* __restri
 #pragma unroll
     for (int k = 0; k < kApplyOrb; ++k) {
       if (k < n) {
-        const int tt = k <= i ? i * (i + 1) / 2 + k : k * (k + 1) / 2 + i;
-        const double re = Vt[2 * tt * RPV + xx], im = Vt[(2 * tt + 1) * RPV + xx];
+        const int hi = max(i, k), lo = min(i, k);
+        double re, im;
+        if (packed) {  // pairs lo < hi, then the real diagonals
+          const int tt = hi * (hi - 1) / 2 + lo;
+          re = Vt[(lo == hi ? n * (n - 1) + lo : 2 * tt) * RPV + xx];
+          im = lo == hi ? 0.0 : Vt[(2 * tt + 1) * RPV + xx];
+        } else {
+          const int tt = hi * (hi + 1) / 2 + lo;
+          re = Vt[2 * tt * RPV + xx];
+          im = Vt[(2 * tt + 1) * RPV + xx];
+        }
         cfma(a, make_double2(re, k <= i ? im : -im), ph[k]);
       }
     }
@@ -956,12 +1174,25 @@ static size_t rp_apply_smem(int n, int NC, int FN) {
   return std::max(stages, epi);
 }
 
-// column fragments per warp (CTA width 16 FN, FN <= 7 for the static shared
-// memory) with the fewest padded columns of NC, the widest on ties
+template <bool HALF, int FN>
+static int launch_rp_dmma(Ctx& c, dim3 grid, const double* Rpl, const double* Wm, const int* d_rows, int K, int NC,
+                          double2* out, const int* d_tmap) {
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      rp_dmma_kernel<HALF, FN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rp_stage_bytes<FN>());
+  SG_CUDA(attr);
+  rp_dmma_kernel<HALF, FN><<<grid, 256, rp_stage_bytes<FN>(), c.stream>>>(Rpl, Wm, d_rows, K, NC, c.G, out, d_tmap,
+                                                                          c.nspf);
+  SG_LAUNCHED();
+  return SINCGPU_OK;
+}
+
+// column fragments per warp (CTA width 16 FN) with the fewest padded columns of NC, the
+// widest on ties; up to 64 columns one narrow tile
 static int rp_dmma_fn(int NC) {
-  int best = 7;
+  if (NC <= 64) return std::max(2, ceil_div(NC, 16));
+  int best = 8;
   long long waste = -1;
-  for (int fn : {7, 6, 5, 4}) {
+  for (int fn : {8, 7, 6, 5, 4}) {
     const long long w = (long long)ceil_div(NC, 16 * fn) * 16 * fn - NC;
     if (waste < 0 || w < waste) {
       waste = w;
@@ -976,28 +1207,36 @@ static int reduced_pot_impl(Ctx& c, const double* Rpl, const int* h_pa, const in
   if (apply) apply->done = false;
   const int n = c.nspf;
   half = half && herm;
-  const int nt = n * (n + 1) / 2;
-  const int K = 2 * npair, NC = half ? 2 * nt : 2 * n * n;
+  const bool packed = half && drop_rows(c, herm) && c.rp_dmma && !c.contract_tf32;
+  std::vector<int> rows, rowof;
+  if (packed) hermitian_rows(h_pa, h_pb, npair, rows, rowof);
+  const int nt = packed ? n * (n - 1) / 2 + (n + 1) / 2 : n * (n + 1) / 2;
+  const int K = packed ? (int)rows.size() : 2 * npair, NC = half ? 2 * nt : 2 * n * n;
   size_t need = sizeof(double) * (size_t)K * NC;
   SG_TRY(c.ws_gemm.ensure(need));
   double* Wm = (double*)c.ws_gemm.ptr;
-  const int *d_pa, *d_pb, *d_tmap = nullptr;
+  const int *d_pa, *d_pb, *d_tmap = nullptr, *d_rows = nullptr;
   SG_TRY(cached_ints(c, IC_PA, h_pa, npair, &d_pa));
   SG_TRY(cached_ints(c, IC_PB, h_pb, npair, &d_pb));
   if (half) {
     std::vector<int> tm;
     tm.reserve(2 * (size_t)nt);
     for (int ii = 0; ii < n; ++ii)
-      for (int kk = 0; kk <= ii; ++kk) {
+      for (int kk = 0; kk <= ii - (packed ? 1 : 0); ++kk) {
         tm.push_back(kk);
         tm.push_back(ii);
       }
-    SG_TRY(cached_ints(c, IC_TMAP, tm.data(), tm.size(), &d_tmap));
+    for (int d = 0; packed && d < n; d += 2) {
+      tm.push_back(-1 - d);
+      tm.push_back(d + 1 < n ? d + 1 : -1);
+    }
+    SG_TRY(cached_ints(c, packed ? IC_TMAP_PACKED : IC_TMAP, tm.data(), tm.size(), &d_tmap));
+    if (packed) SG_TRY(cached_ints(c, IC_RROWS, rows.data(), rows.size(), &d_rows));
   }
   {
     ProfScope ps(c, ST_RP_W);
     if (half)
-      build_w_half_kernel<<<ceil_div((long long)K * NC, 256), 256, 0, c.stream>>>(tally, d_pa, d_pb, d_tmap,
+      build_w_half_kernel<<<ceil_div((long long)K * NC, 256), 256, 0, c.stream>>>(tally, d_pa, d_pb, d_tmap, d_rows, K,
                                                                                   npair, n, nt, Wm);
     else
       build_w_kernel<<<ceil_div((long long)K * NC, 256), 256, 0, c.stream>>>(tally, d_pa, d_pb, npair, n,
@@ -1020,11 +1259,12 @@ static int reduced_pot_impl(Ctx& c, const double* Rpl, const int* h_pa, const in
   if (c.rp_dmma) {
     const int fn = rp_dmma_fn(NC);
     const dim3 grid((unsigned)ceil_div(c.G, DM), (unsigned)ceil_div(NC, 16 * fn));
-    // one column tile (n(n+1) <= 112, so n <= 10: the epilogue's per-thread orbital registers)
-    if (apply && half && grid.y == 1 && n <= 10) {
+    // one column tile of at most 112 columns and n <= 10 (the epilogue's per-thread orbital registers)
+    if (apply && half && grid.y == 1 && fn <= 7 && n <= 10) {
       // process-wide attributes, one fixed value each (thread-safe static initialisation)
       static const cudaError_t attr = [] {
-        const void* ks[] = {(const void*)rp_apply_kernel<4>, (const void*)rp_apply_kernel<5>,
+        const void* ks[] = {(const void*)rp_apply_kernel<2>, (const void*)rp_apply_kernel<3>,
+                            (const void*)rp_apply_kernel<4>, (const void*)rp_apply_kernel<5>,
                             (const void*)rp_apply_kernel<6>, (const void*)rp_apply_kernel<7>};
         for (const void* k : ks) {
           const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1038,10 +1278,13 @@ static int reduced_pot_impl(Ctx& c, const double* Rpl, const int* h_pa, const in
       const size_t sm = rp_apply_smem(n, NC, fn);
 #define SG_RP_APPLY(FN)                                                                                  \
   case FN:                                                                                               \
-    rp_apply_kernel<FN><<<grid, 256, sm, c.stream>>>(Rpl, Wm, K, NC, c.G, reducedpot, d_tmap, n, apply->phi, \
-                                                     apply->S, apply->inv, apply->timefac, apply->T);    \
+    rp_apply_kernel<FN><<<grid, 256, sm, c.stream>>>(Rpl, Wm, d_rows, packed ? 1 : 0, K, NC, c.G, reducedpot, \
+                                                     d_tmap, n, apply->phi, apply->S, apply->inv, apply->timefac,      \
+                                                     apply->T);                                            \
     break;
       switch (fn) {
+        SG_RP_APPLY(2)
+        SG_RP_APPLY(3)
         SG_RP_APPLY(4)
         SG_RP_APPLY(5)
         SG_RP_APPLY(6)
@@ -1053,22 +1296,22 @@ static int reduced_pot_impl(Ctx& c, const double* Rpl, const int* h_pa, const in
       apply->done = true;
       return SINCGPU_OK;
     }
-#define SG_RP_DMMA(FN)                                                                                   \
-  case FN:                                                                                               \
-    if (half)                                                                                            \
-      rp_dmma_kernel<true, FN><<<grid, 256, 0, c.stream>>>(Rpl, Wm, K, NC, c.G, reducedpot, d_tmap, n);  \
-    else                                                                                                 \
-      rp_dmma_kernel<false, FN><<<grid, 256, 0, c.stream>>>(Rpl, Wm, K, NC, c.G, reducedpot, nullptr, n); \
+#define SG_RP_DMMA(FN)                                                          \
+  case FN:                                                                      \
+    SG_TRY((half ? launch_rp_dmma<true, FN>(c, grid, Rpl, Wm, d_rows, K, NC, reducedpot, d_tmap) \
+                 : launch_rp_dmma<false, FN>(c, grid, Rpl, Wm, nullptr, K, NC, reducedpot, nullptr))); \
     break;
     switch (fn) {
+      SG_RP_DMMA(2)
+      SG_RP_DMMA(3)
       SG_RP_DMMA(4)
       SG_RP_DMMA(5)
       SG_RP_DMMA(6)
+      SG_RP_DMMA(7)
       default:
-        SG_RP_DMMA(7)
+        SG_RP_DMMA(8)
     }
 #undef SG_RP_DMMA
-    SG_LAUNCHED();
     return SINCGPU_OK;
   }
   const int gx = ceil_div(c.G, RM);
