@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <vector>
 #include "context.hpp"
+#include "dmma.cuh"
 
 namespace sincgpu {
 
@@ -40,14 +41,6 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool va
   int n = valid ? 16 : 0;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(n));
 }
-// D (8 x 8, two values per lane) += A (8 x 4) B (4 x 8) on the FP64 tensor cores;
-// lane g * 4 + t holds A[g][t], B[t][g] and D[g][2t], D[g][2t + 1]
-__device__ __forceinline__ void dmma_884(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
-
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }

@@ -596,33 +596,39 @@ __global__ void lv_add_kernel(double2* __restrict__ a, const double2* __restrict
 // S^(-1/2) of the overlap by SVD with singular values below 1e-10 dropped
 // (symorthogmat, MCTDH.SRC/utils.f90:947-1023: out = U diag(f(s)) V^H), and
 // the orthonormality error max|S - 1| of the overlap on input.
-__global__ void __launch_bounds__(32) orthogmat_kernel(const double2* __restrict__ S_in, int n,
-                                                       double2* __restrict__ out, double* __restrict__ err) {
+// 16 warps: the rotations of a round of the SVD side by side (one warp took 111 us at 10
+// orbitals, 29 now; 57 and 19 at 8).
+constexpr int kOrthoThreads = 512;
+__global__ void __launch_bounds__(kOrthoThreads) orthogmat_kernel(const double2* __restrict__ S_in, int n,
+                                                                  double2* __restrict__ out,
+                                                                  double* __restrict__ err) {
   __shared__ double2 A[32 * 32], V[32 * 32];
-  __shared__ double sv[32];
-  const int k = threadIdx.x;
-  double e = 0.0;
-  if (k < n)
-    for (int j = 0; j < n; ++j) {
-      double2 d = S_in[k + n * j];
-      if (k == j) d.x -= 1.0;
-      e = fmax(e, sqrt(d.x * d.x + d.y * d.y));
-    }
-  for (int o = 16; o > 0; o >>= 1) e = fmax(e, __shfl_xor_sync(0xffffffffu, e, o));
-  if (k == 0 && err) *err = e;
+  __shared__ double sv[32], f[32];
+  const int k = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (w == 0) {
+    double e = 0.0;
+    if (k < n)
+      for (int j = 0; j < n; ++j) {
+        double2 d = S_in[k + n * j];
+        if (k == j) d.x -= 1.0;
+        e = fmax(e, sqrt(d.x * d.x + d.y * d.y));
+      }
+    for (int o = 16; o > 0; o >>= 1) e = fmax(e, __shfl_xor_sync(0xffffffffu, e, o));
+    if (k == 0 && err) *err = e;
+  }
   if (!out) return;
-  hestenes_svd_warp(S_in, n, A, V, sv);
+  hestenes_svd_block(S_in, n, A, V, sv);
+  if (w == 0 && k < n) f[k] = sv[k] < 1e-10 ? 0.0 : 1.0 / sqrt(sv[k]) / sv[k];
+  __syncthreads();
   // out(i,j) = sum_m U(i,m) f(s_m) conj(V(j,m)),  U(i,m) = A(i,m) / s_m
-  if (k < n)
-    for (int j = 0; j < n; ++j) {
+  for (int j = w; j < n; j += kOrthoThreads / 32)
+    if (k < n) {
       double2 acc = make_double2(0.0, 0.0);
       for (int m = 0; m < n; ++m) {
-        const double s = sv[m];
-        if (s < 1e-10) continue;
-        const double f = 1.0 / sqrt(s) / s;
+        if (sv[m] < 1e-10) continue;
         const double2 t = cmulc(A[k + 32 * m], V[j + 32 * m]);  // A(i,m) conj(V(j,m))
-        acc.x = fma(f, t.x, acc.x);
-        acc.y = fma(f, t.y, acc.y);
+        acc.x = fma(f[m], t.x, acc.x);
+        acc.y = fma(f[m], t.y, acc.y);
       }
       out[k + n * j] = acc;
     }
@@ -747,7 +753,7 @@ int spf_orthogit(Ctx& c, double2* phi, double* error) {
   const long long nv = c.G * n;
   for (int ii = 0; ii < 3; ++ii) {
     SG_TRY(orbital_dots(c, phi, phi, o.ovl, o.dpart));
-    orthogmat_kernel<<<1, 32, 0, c.stream>>>(o.ovl, n, ii < 2 ? o.smh : nullptr, o.err);
+    orthogmat_kernel<<<1, kOrthoThreads, 0, c.stream>>>(o.ovl, n, ii < 2 ? o.smh : nullptr, o.err);
     SG_LAUNCHED();
     if (ii < 2) {
       SG_TRY(orbital_mix(c, phi, o.smh, o.tmp));

@@ -16,18 +16,13 @@
 // memory, so no thread keeps an n-vector in registers.
 #include <algorithm>
 #include "context.hpp"
+#include "dmma.cuh"
 
 namespace sincgpu {
 
 constexpr int TXO = 32;          // grid points per tile (lanes)
 constexpr int kMaxOrbRhs = 32;   // largest orbital count of these kernels
 constexpr int kRhsSmemMax = 64 * 1024;
-
-__device__ __forceinline__ void dmma_884(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
 
 // out(x,i) = [base(x,i)] + sgn sum_s sum_j src_s(x,j) mat_s(j,i), s < NS (column-major n x n
 // complex matrices): the mix with denmat or an overlap's root, the projection and the
