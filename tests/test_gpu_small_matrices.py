@@ -60,3 +60,32 @@ def test_orthogonalisation(built_lib, n):
     assert np.abs(out - ref).max() < 1e-12
     assert np.abs(np.conj(out).T @ out - np.eye(n)).max() < 1e-12
     assert err == pytest.approx(err_ref, abs=1e-12)
+
+
+# 784 determinants: four warps a configuration; 3025: one; 14400: the general kernel, and
+# vectors whose rows beyond the eleventh stay outside shared memory
+@pytest.mark.parametrize("numelec,n,m", [(4, 8, 20), (4, 11, 20), (4, 16, 18)])
+def test_krylov_forms(built_lib, numelec, n, m):
+    from sincgpu import SincProject, WalkTables
+    sysm = orc.SincSystem(9, 0.5, [[0, 0, 0]], [2.0])
+    with SincProject(9, 0.5, [[0, 0, 0]], [2.0], n) as gpu:
+        walks = WalkTables(numelec, n, 0)
+        nc = walks.numconfig
+        gpu.ci_attach(walks)
+        phi = orc.seeded_orbitals(sysm, n, seed=5)
+        rng = np.random.default_rng(6)
+        mat = rng.standard_normal((n,) * 4) + 1j * rng.standard_normal((n,) * 4)
+        mat = (mat + np.conj(mat.transpose(2, 3, 0, 1))) / n
+        ph = np.conj(phi).T
+        gpu.assemble_sparsemats(np.asfortranarray(mat), ph @ sysm.mult_pot(phi), ph @ sysm.mult_ke(phi),
+                                ph @ sysm.mult_zdipole(phi))
+        a = rng.standard_normal(nc) + 1j * rng.standard_normal(nc)
+        a /= np.linalg.norm(a)
+        outs = []
+        for cluster in (1, 0):
+            gpu.set_option("kry_cluster", cluster)
+            outs.append(gpu.expoavecprop(a, 1.0, krylovdim=m, tol=1e-10, anorm=0.02, stepguess=1.0, timefac=-0.02j,
+                                         ezfield=0.1))
+        assert outs[0][2] == outs[1][2]
+        # two roundings of the same recurrence, as test_matrix_exponential
+        assert np.abs(outs[0][0] - outs[1][0]).max() < 1e-10

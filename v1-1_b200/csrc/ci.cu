@@ -598,14 +598,135 @@ __global__ void __launch_bounds__(128) sigma_kernel(const long long* __restrict_
   }
 }
 
+// hop_sum over [h, e) in steps of D, the first U matrix elements and targets loaded by load()
+template <int U, int D>
+struct HopSum {
+  long long h, e;
+  int t[U];
+  double2 m[U];
+  template <class MAT>
+  __device__ __forceinline__ void load(const int* __restrict__ hop, const MAT& mat) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool ok = h + D * u < e;
+      t[u] = ok ? __ldcs(hop + h + D * u) : -1;
+      m[u] = ok ? mat(h + D * u) : make_double2(0.0, 0.0);
+    }
+  }
+  template <class MAT>
+  __device__ __forceinline__ double2 sum(const int* __restrict__ hop, const MAT& mat, const double2* a) {
+    double2 acc = make_double2(0.0, 0.0);
+    while (h < e) {
+      double2 v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = t[u] >= 0 ? a[t[u]] : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (t[u] >= 0) acc = cadd(acc, cmul(m[u], v[u]));
+      h += D * U;
+      if (h < e) load(hop, mat);
+    }
+    return acc;
+  }
+};
+
+// The same sum for a small space, whose time is the latency of one row's loads: all warps are
+// resident at once (24 an SM), a row's first 256 two-electron elements are loaded together,
+// by W warps, and before the wait for the kernel in front, which may write `in` and *skip.
+// 3136 determinants in a Krylov chain: 4.4 us from the wait to the end where the general
+// kernel took some 10 with its launch.
+constexpr int kSigmaWarps = 148 * 24;
+template <int W>
+__global__ void __launch_bounds__(128, 6) sigma_small_kernel(const long long* __restrict__ doff,
+                                                             const int* __restrict__ dhop,
+                                                             const double2* __restrict__ xpot,
+                                                             const long long* __restrict__ soff,
+                                                             const int* __restrict__ shop,
+                                                             const double2* __restrict__ xone,
+                                                             const double2* __restrict__ xz, double ez, double diag,
+                                                             const double2* in, int nc, double2* out, double2 tf,
+                                                             int scaled, const int* skip) {
+  __shared__ double2 part[4];
+  const int warp = threadIdx.x >> 5, l = threadIdx.x % (32 * W);
+  const int c1 = blockIdx.x * (4 / W) + warp / W;
+  const bool ok = c1 < nc;
+  auto two = [&](long long h) { return __ldcs(xpot + h); };
+  auto one = [&](long long h) {
+    double2 m = xone ? __ldcs(xone + h) : make_double2(0.0, 0.0);
+    if (ez != 0.0) {
+      const double2 z = __ldcs(xz + h);
+      m.x = fma(ez, z.x, m.x);
+      m.y = fma(ez, z.y, m.y);
+    }
+    return m;
+  };
+  HopSum<8 / W, 32 * W> d;
+  HopSum<1, 32 * W> s;
+  d.h = d.e = s.h = s.e = 0;
+  if (ok) {
+    if (xpot) {
+      d.h = doff[c1] + l;
+      d.e = doff[c1 + 1];
+    }
+    s.h = soff[c1] + l;
+    s.e = soff[c1 + 1];
+  }
+  d.load(dhop, two);
+  s.load(shop, one);
+  grid_dependents_launch();
+  grid_dependency_wait();
+  if (skip && *skip) return;
+  double2 acc = warp_sum(cadd(d.sum(dhop, two, in), s.sum(shop, one, in)));
+  if (W > 1) {
+    if ((threadIdx.x & 31) == 0) part[warp] = acc;
+    __syncthreads();
+  }
+  if (l == 0 && ok) {
+    const double2 a = in[c1];
+    double2 r = make_double2(diag * a.x, diag * a.y);
+    if (W > 1) {
+#pragma unroll
+      for (int w = 0; w < W; ++w) r = cadd(r, part[warp + w]);
+    } else {
+      r = cadd(r, acc);
+    }
+    out[c1] = scaled ? cmul(tf, r) : r;
+  }
+}
+
+// `early`: a small space's kernel may start before the one in front has ended
+static int launch_sigma(Ctx& c, bool early, const double2* xpot, const double2* xone, double ez, double diag,
+                        const double2* in, double2* out, double2 tf, bool scaled, const int* skip) {
+  CIState& s = c.ci;
+  if (s.nc > kSigmaWarps) {
+    sigma_kernel<<<ceil_div(s.nc, 4), 128, 0, c.stream>>>(s.dhop_off, s.dhop, xpot, s.shop_off, s.shop, xone, s.xz, ez,
+                                                          diag, in, s.nc, out, tf, scaled ? 1 : 0, skip);
+    SG_LAUNCHED();
+    return SINCGPU_OK;
+  }
+  const bool four = s.nc <= kSigmaWarps / 4;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ceil_div(s.nc, four ? 1 : 4), 1, 1);
+  cfg.blockDim = dim3(128, 1, 1);
+  cfg.stream = c.stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = early ? 1 : 0;
+  SG_CUDA(cudaLaunchKernelEx(&cfg, four ? sigma_small_kernel<4> : sigma_small_kernel<1>, (const long long*)s.dhop_off,
+                             (const int*)s.dhop, xpot, (const long long*)s.shop_off, (const int*)s.shop, xone,
+                             (const double2*)s.xz, ez, diag, in, s.nc, out, tf, scaled ? 1 : 0, skip));
+  count_launch();
+  return SINCGPU_OK;
+}
+
 // z-dipole expectation (dipolesub_one, MCTDH.SRC/dipolesub.f90:20-125, z part):
 // <A| Z A> with Z the singles of <phi_i|z|phi_j>, plus nucdip <A|A>; also <A|A>
 int ci_dipole_z(Ctx& c, const double2* a, double2* tmp, double nucdipz, double2* dip, double* normsq) {
   CIState& s = c.ci;
   SG_CHECK(s.attached && s.assembled, SINCGPU_ESTATE, "sparse CI matrices not assembled");
-  sigma_kernel<<<ceil_div(s.nc, 4), 128, 0, c.stream>>>(s.dhop_off, s.dhop, nullptr, s.shop_off, s.shop, nullptr,
-                                                        s.xz, 1.0, 0.0, a, s.nc, tmp, make_double2(1.0, 0.0), 0, nullptr);
-  SG_LAUNCHED();
+  SG_TRY(launch_sigma(c, false, nullptr, nullptr, 1.0, 0.0, a, tmp, make_double2(1.0, 0.0), false, nullptr));
   std::vector<double2> ha(s.nc), za(s.nc);
   SG_CUDA(cudaMemcpyAsync(ha.data(), a, sizeof(double2) * s.nc, cudaMemcpyDeviceToHost, c.stream));
   SG_CUDA(cudaMemcpyAsync(za.data(), tmp, sizeof(double2) * s.nc, cudaMemcpyDeviceToHost, c.stream));
@@ -632,11 +753,9 @@ int ci_sigma(Ctx& c, const double2* in, double2* out, double constant, double ez
   CIState& s = c.ci;
   SG_CHECK(s.attached && s.assembled, SINCGPU_ESTATE, "sparse CI matrices not assembled");
   ProfScope ps(c, ST_CI);
-  sigma_kernel<<<ceil_div(s.nc, 4), 128, 0, c.stream>>>(s.dhop_off, s.dhop, s.xpot, s.shop_off, s.shop, s.xone,
-                                                        s.xz, ez, constant + ez * nucdipz, in, s.nc, out, tf,
-                                                        skip ? 1 : 0, skip);
-  SG_LAUNCHED();
-  return SINCGPU_OK;
+  // in a Krylov chain the kernel in front writes `in` and the flag
+  return launch_sigma(c, skip != nullptr, s.xpot, s.xone, ez, constant + ez * nucdipz, in, out, tf, skip != nullptr,
+                      skip);
 }
 
 }  // namespace sincgpu

@@ -55,6 +55,12 @@ __host__ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 #ifdef __CUDACC__
+// Launched with programmatic stream serialization a kernel may start before the one in front
+// of it has ended: what that one writes is read only after the wait (both are no-ops in an
+// ordinary launch).
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// the kernel behind may start once every CTA has come here
+__device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;"); }
 // acc += v*m with explicit FMAs (one rounding order wherever it is used)
 __device__ __forceinline__ void cfma(double2& acc, double2 v, double2 m) {
   acc.x = fma(v.x, m.x, fma(-v.y, m.y, acc.x));

@@ -102,118 +102,185 @@ __global__ void __launch_bounds__(kKryThreads) kry_mgs_kernel(double* __restrict
 // formed in the same pass over V (v_j is a row already) and kept for later steps.
 //
 // CTA q of the cluster owns the slice [q S, q S + S) of the vectors, S = ceil(n /
-// kGsCluster) rounded up to even; p and v_j of the slice sit in shared memory.  Warp w
-// sums the dots of rows w, w + 32, ...; the CTAs' partials are added in rank order
-// through distributed shared memory, so every CTA gets the same value.
-// What bounds it: the latency of four dependent stages (loads of p, dots, update, norm)
-// and two cluster barriers, 12 to 14 us a step with cold caches, against j + 2
-// dependent sums in one CTA (784 determinants, 30 vectors: 21.9 us a step) or over the
-// cluster (3136 determinants: 32.6 us).  One A-vector step of 30 vectors at 3136
-// determinants: 1627 -> 901 us, with the sigma product's scaling folded in and the
-// cluster form of the update (94 -> 20 us).
-constexpr int kGsCluster = 8;
-constexpr long long kGsSlice = 14080;  // values of a slice: p and v_j in 220 KB
+// kGsCluster) rounded up to even; p, v_j and the first `cap` rows of the slice sit in
+// shared memory (all of them for 30 vectors up to some 5,800 determinants), further rows
+// come from L2.  A warp sums up to four rows over half the slice; the CTAs' partials are added
+// in a fixed order through distributed shared memory, so every CTA gets the same value.
+// What bounds it: the latency of its dependent stages (load of p, dots, update, norm) and
+// two cluster barriers.  The rows' way into shared memory comes before the wait for the
+// sigma product that writes p: that product and the step before may still run (512
+// threads, so that all fit an SM).  After the wait, at 25 rows of 3136 determinants: loads
+// 0.8 us, dots 2.2, barrier 0.7, coefficients 1.1, update 0.9, norm 1.2.  One A-vector step
+// of 30 vectors at 3136 determinants, launches included: 810 -> 515 us, of which clusters of
+// 8 whose rows came from L2 after the sigma product had ended took 14 us a vector; CMF step
+// at 31^3 14.3 -> 12.1 ms.
+constexpr int kGsCluster = 16;
+constexpr int kGsThreads = 32 * kGsCluster;
+constexpr long long kGsSlice = 8100;    // most values of a slice
+constexpr long long kGsValues = 23900;  // of dynamic shared memory: p, v_j, rows of L, rows of V
+static_assert(2 * kGsSlice + kMaxKry * (kMaxKry - 1) / 2 <= kGsValues, "p, v_j and L must fit");
 
-__global__ void __launch_bounds__(kKryThreads) kry_gs_kernel(double* __restrict__ V, long long n, int S, int j,
-                                                             double* __restrict__ Hm, int mh,
-                                                             double* __restrict__ Lm, double break_tol, KryState* st) {
+__device__ __forceinline__ void cp_async16(double* smem, const double* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem));
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+// out[half][i] = (<v, x>, <v, y>) with v = row(i) over the warp's half of the slice, for the NR
+// rows i0, i0 + 8, .. (the last row for those past it); the lanes' sums change places as
+// they are halved, so that 2 NR values take 2 NR + 1 or so exchanges instead of 10 NR
+template <int NR, class Row>
+__device__ __forceinline__ void gs_dots(int i0, int last, int half, int len, const double* x, const double* y, Row row,
+                                        double2 (*out)[128]) {
+  const int lane = threadIdx.x & 31;
+  const double* v[NR];
+  double a[2 * NR];
+#pragma unroll
+  for (int u = 0; u < NR; ++u) {
+    v[u] = row(min(i0 + 8 * u, last));
+    a[2 * u] = a[2 * u + 1] = 0.0;
+  }
+#pragma unroll 4
+  for (int k = 32 * half + lane; k < len; k += 64) {
+    const double xk = x[k], yk = y[k];
+#pragma unroll
+    for (int u = 0; u < NR; ++u) {
+      const double vk = v[u][k];
+      a[2 * u] = fma(vk, xk, a[2 * u]);
+      a[2 * u + 1] = fma(vk, yk, a[2 * u + 1]);
+    }
+  }
+  int which = 0;
+#pragma unroll
+  for (int o = 16, c = NR; o > 0; o >>= 1, c >>= 1) {
+    if (c > 0) {  // keep c of the 2 c values left
+      const bool up = lane & o;
+#pragma unroll
+      for (int u = 0; u < c; ++u) {
+        const double give = up ? a[u] : a[u + c], keep = up ? a[u + c] : a[u];
+        a[u] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+      if (up) which += c;
+    } else {
+      a[0] += __shfl_xor_sync(0xffffffffu, a[0], o);
+    }
+  }
+  const int i = i0 + 8 * (which >> 1);
+  if (lane % (16 / NR) == 0 && i <= last) (which & 1 ? out[half][i].y : out[half][i].x) = a[0];
+}
+
+// ALL: cap = j, every row in shared memory
+template <bool ALL>
+__global__ void __launch_bounds__(kGsThreads) kry_gs_kernel(double* V, long long n, int S, int cap, int j,
+                                                            double* Hm, int mh, double* Lm, double break_tol,
+                                                            KryState* st) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
-  extern __shared__ double gsm[];  // p slice, v_j slice
-  __shared__ double red[33];
-  __shared__ double part[2][128];  // this CTA's partial dots <v_i, p>, <v_i, v_j>
-  __shared__ double npart, r[128], lrow[128], h[128];
-  if (st->mbrk) return;  // the same value in every CTA of the cluster
+  extern __shared__ __align__(16) double gsm[];  // p, v_j, rows 0 .. cap - 1 of the slice, rows of L
+  __shared__ double2 part[kGsCluster][128];  // every CTA's partial dots <v_i, p>, <v_i, v_j>
+  __shared__ double2 dots[2][128];           // this CTA's, by halves of its slice
+  __shared__ double npart[kGsCluster], red[kGsThreads / 32], r[128], lrow[128], h[128];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const long long lo = (long long)cl.block_rank() * S;
+  const int rank = cl.block_rank();
+  const long long lo = (long long)rank * S;
   const int len = (int)max(0LL, min((long long)S, n - lo));
   double* ps = gsm;
-  double* vs = gsm + S;
-  const double* vj = V + (long long)j * n + lo;
+  double* Ls = gsm + (long long)(2 + cap) * S;  // row i from i (i - 1) / 2
   double* pg = V + (long long)(j + 1) * n + lo;
-  for (int k = tid; k < len; k += kKryThreads) {
-    ps[k] = pg[k];
-    vs[k] = vj[k];
+  auto row = [&](int i) -> const double* {
+    if (ALL) return gsm + (i == j ? 1 : 2 + i) * S;
+    return i == j ? gsm + S : i < cap ? gsm + (long long)(2 + i) * S : V + (long long)i * n + lo;
+  };
+  // Before the wait: rows 0 .. j - 1 of V and 0 .. j - 2 of L, all of steps that have ended
+  // (the step in front waits for its own predecessor before it lets this one start).
+  // Rows as pairs: n, S and so every len are even.
+  for (int i = warp; i < cap; i += kGsThreads / 32)
+    for (int k = 2 * lane; k < len; k += 64)
+      cp_async16(gsm + (long long)(2 + i) * S + k, V + (long long)i * n + lo + k);
+  for (int i = warp; i < j - 1; i += kGsThreads / 32)
+    for (int k = lane; k < i; k += 32) Ls[i * (i - 1) / 2 + k] = __ldcg(Lm + (long long)i * mh + k);
+  cp_async_wait_all();
+  cl.sync();  // the CTAs whose shared memory is written are there
+  grid_dependency_wait();
+  grid_dependents_launch();
+  const int brk_before = *(volatile int*)&st->mbrk;  // the same value in every CTA
+  const double* vj = V + (long long)j * n + lo;
+  for (int k = tid; k < len; k += kGsThreads) {
+    ps[k] = __ldcg(pg + k);
+    gsm[S + k] = __ldcg(vj + k);
+  }
+  if (tid < j - 1) Ls[(j - 1) * (j - 2) / 2 + tid] = __ldcg(Lm + (long long)(j - 1) * mh + tid);
+  __syncthreads();
+  if (brk_before) return;
+  for (int base = 0; base <= j; base += 32) {
+    const int i0 = base + (warp & 7), left = j + 1 - base;
+    if (left > 16) gs_dots<4>(i0, j, warp >> 3, len, ps, gsm + S, row, dots);
+    else if (left > 8) gs_dots<2>(i0, j, warp >> 3, len, ps, gsm + S, row, dots);
+    else gs_dots<1>(i0, j, warp >> 3, len, ps, gsm + S, row, dots);
   }
   __syncthreads();
-  for (int i = warp; i <= j; i += kKryThreads / 32) {
-    const double* vi = V + (long long)i * n + lo;
-    double a = 0.0, b = 0.0;
-    int k = lane;
-    for (; k + 96 < len; k += 128) {
-      const double v0 = vi[k], v1 = vi[k + 32], v2 = vi[k + 64], v3 = vi[k + 96];
-      a = fma(v3, ps[k + 96], fma(v2, ps[k + 64], fma(v1, ps[k + 32], fma(v0, ps[k], a))));
-      b = fma(v3, vs[k + 96], fma(v2, vs[k + 64], fma(v1, vs[k + 32], fma(v0, vs[k], b))));
-    }
-    for (; k < len; k += 32) {
-      const double v = vi[k];
-      a = fma(v, ps[k], a);
-      b = fma(v, vs[k], b);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      a += __shfl_down_sync(0xffffffffu, a, o);
-      b += __shfl_down_sync(0xffffffffu, b, o);
-    }
-    if (lane == 0) {
-      part[0][i] = a;
-      part[1][i] = b;
-    }
-  }
+  static_assert(kGsThreads / 32 == kGsCluster, "a warp per CTA of the cluster");
+  for (int i = lane; i <= j; i += 32) *cl.map_shared_rank(&part[rank][i], warp) = cadd(dots[0][i], dots[1][i]);
   cl.sync();
   if (tid <= j) {
-    double a = 0.0, b = 0.0;
+    double2 a[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
 #pragma unroll
-    for (int q = 0; q < kGsCluster; ++q) {
-      const double* o = cl.map_shared_rank(&part[0][0], q);
-      a += o[tid];
-      b += o[128 + tid];
-    }
-    r[tid] = a;
-    // row j of L (its diagonal is not used)
-    if (cl.block_rank() == 0 && tid < j) Lm[(long long)j * mh + tid] = b;
-    lrow[tid] = b;
+    for (int q = 0; q < kGsCluster; ++q) a[q & 1] = cadd(a[q & 1], part[q][tid]);
+    const double2 sum = cadd(a[0], a[1]);
+    r[tid] = sum.x;
+    lrow[tid] = sum.y;  // row j of L (its diagonal is not used)
+    if (rank == 0 && tid < j) Lm[(long long)j * mh + tid] = sum.y;
   }
   __syncthreads();
   // h_i = r_i - sum_{k < i} L_ik r_k, a warp per row, the same in every CTA
-  for (int i = warp; i <= j; i += kKryThreads / 32) {
+  for (int i = warp; i <= j; i += kGsThreads / 32) {
+    const double* L = i < j ? Ls + i * (i - 1) / 2 : lrow;
     double a = 0.0;
-    for (int k = lane; k < i; k += 32) a = fma(i < j ? Lm[(long long)i * mh + k] : lrow[k], r[k], a);
+    for (int k = lane; k < i; k += 32) a = fma(L[k], r[k], a);
     for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
     if (lane == 0) {
       h[i] = r[i] - a;
-      if (cl.block_rank() == 0) Hm[(long long)j * mh + i] = r[i] - a;
+      if (rank == 0) Hm[(long long)j * mh + i] = r[i] - a;
     }
   }
   __syncthreads();
   double s = 0.0;
-  for (int k = tid; k < len; k += kKryThreads) {
-    const double* vk = V + lo + k;
-    double x = ps[k];
+  const int staged = ALL ? j : cap;
+  for (int k = tid; k < len; k += kGsThreads) {
+    double x[4] = {fma(-h[j], gsm[S + k], ps[k]), 0.0, 0.0, 0.0};
     int i = 0;
-    for (; i + 3 <= j; i += 4) {
-      const double v0 = vk[(long long)i * n], v1 = vk[(long long)(i + 1) * n], v2 = vk[(long long)(i + 2) * n],
-                   v3 = vk[(long long)(i + 3) * n];
-      x = fma(-h[i + 3], v3, fma(-h[i + 2], v2, fma(-h[i + 1], v1, fma(-h[i], v0, x))));
-    }
-    for (; i <= j; ++i) x = fma(-h[i], vk[(long long)i * n], x);
-    ps[k] = x;
-    s = fma(x, x, s);
+#pragma unroll 2
+    for (; i + 4 <= staged; i += 4)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) x[u] = fma(-h[i + u], gsm[(2 + i + u) * S + k], x[u]);
+    for (; i < staged; ++i) x[0] = fma(-h[i], gsm[(2 + i) * S + k], x[0]);
+    for (; !ALL && i + 4 <= j; i += 4)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) x[u] = fma(-h[i + u], V[(long long)(i + u) * n + lo + k], x[u]);
+    for (; !ALL && i < j; ++i) x[0] = fma(-h[i], V[(long long)i * n + lo + k], x[0]);
+    x[0] += x[1] + (x[2] + x[3]);
+    ps[k] = x[0];
+    s = fma(x[0], x[0], s);
   }
-  s = block_sum(s, red);
-  if (tid == 0) npart = s;
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) red[warp] = s;
+  __syncthreads();
+  if (warp == 0) {
+    s = lane < kGsThreads / 32 ? red[lane] : 0.0;
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane < kGsCluster) *cl.map_shared_rank(&npart[rank], lane) = s;
+  }
   cl.sync();
   double t = 0.0;
 #pragma unroll
-  for (int q = 0; q < kGsCluster; ++q) t += *cl.map_shared_rank(&npart, q);
+  for (int q = 0; q < kGsCluster; ++q) t += npart[q];
   const double hn = sqrt(t);
   const bool brk = hn <= break_tol;
-  if (cl.block_rank() == 0 && tid == 0) {
+  if (rank == 0 && tid == 0) {
     if (brk) st->mbrk = j + 1;
     else Hm[(long long)j * mh + j + 1] = hn;
   }
   const double inv = 1.0 / hn;
-  for (int k = tid; k < len; k += kKryThreads) pg[k] = brk ? ps[k] : ps[k] * inv;
-  cl.sync();  // no CTA leaves while another may still read its partials
+  for (int k = tid; k < len; k += kGsThreads) pg[k] = brk ? ps[k] : ps[k] * inv;
 }
 
 // w = beta * V[0:mx]^T exph[0:mx]; beta <- |w|, over the same cluster and slices
@@ -252,21 +319,24 @@ __global__ void __launch_bounds__(kKryThreads) kry_update_cluster_kernel(const d
   cl.sync();  // no CTA leaves while its partial is read
 }
 
-// launch of a kernel on one cluster of kGsCluster CTAs
+// launch of a kernel on one cluster of kGsCluster CTAs; `early`: before the kernel in front
+// of it has ended
 template <class... KA, class... A>
-static int launch_gs_cluster(Ctx& c, void (*kernel)(KA...), size_t smem, A... args) {
+static int launch_gs_cluster(Ctx& c, void (*kernel)(KA...), int threads, size_t smem, bool early, A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(kGsCluster, 1, 1);
-  cfg.blockDim = dim3(kKryThreads, 1, 1);
+  cfg.blockDim = dim3(threads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = c.stream;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = kGsCluster;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = early ? 2 : 1;
   SG_CUDA(cudaLaunchKernelEx(&cfg, kernel, (KA)args...));
   count_launch();
   return SINCGPU_OK;
@@ -510,8 +580,14 @@ int expv_avector(Ctx& c, const double2* v, double2* w, double t, double2 timefac
   // the cluster kernels where a slice of p and v_j fits shared memory, else one CTA
   const long long S = ((n + kGsCluster - 1) / kGsCluster + 1) / 2 * 2;
   const bool cluster = c.kry_cluster && S <= kGsSlice;
-  static const cudaError_t attr = cudaFuncSetAttribute(kry_gs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       (int)(sizeof(double) * 2 * kGsSlice));
+  static const cudaError_t attr = [] {  // fixed values, set once
+    for (auto k : {kry_gs_kernel<true>, kry_gs_kernel<false>}) {
+      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(double) * kGsValues));
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (e != cudaSuccess) return e;
+    }
+    return cudaFuncSetAttribute(kry_update_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  }();
   SG_CUDA(attr);
   while (t_now < t_out) {
     ++nstep;
@@ -525,8 +601,10 @@ int expv_avector(Ctx& c, const double2* v, double2* w, double t, double2 timefac
       SG_TRY(ci_sigma(c, (const double2*)(V + (size_t)j * n), (double2*)(V + (size_t)(j + 1) * n), c.nucrepulsion, ez,
                       nucdipz, timefac, &dst->mbrk));
       if (cluster) {
-        SG_TRY(launch_gs_cluster(c, kry_gs_kernel, sizeof(double) * 2 * (size_t)S, V, n, (int)S, j, Hm, mh, Lm,
-                                 break_tol, dst));
+        const long long tri = j * (j - 1) / 2;
+        const int cap = (int)std::min<long long>(j, (kGsValues - tri) / S - 2);
+        SG_TRY(launch_gs_cluster(c, cap == j ? kry_gs_kernel<true> : kry_gs_kernel<false>, kGsThreads, sizeof(double) * ((2 + cap) * (size_t)S + tri), true, V,
+                                 n, (int)S, cap, j, Hm, mh, Lm, break_tol, dst));
       } else {
         kry_mgs_kernel<<<1, kKryThreads, 0, c.stream>>>(V, n, j, Hm, mh, break_tol, dst);
         SG_LAUNCHED();
@@ -580,7 +658,7 @@ int expv_avector(Ctx& c, const double2* v, double2* w, double t, double2 timefac
     }
     const int mxu = mbrkdwn + std::max(0, k1 - 1);
     if (cluster) {
-      SG_TRY(launch_gs_cluster(c, kry_update_cluster_kernel, 0, V, n, (int)S, mxu, exph, (double*)w, dst));
+      SG_TRY(launch_gs_cluster(c, kry_update_cluster_kernel, kKryThreads, 0, false, V, n, (int)S, mxu, exph, (double*)w, dst));
     } else {
       kry_update_kernel<<<1, kKryThreads, 0, c.stream>>>(V, n, mxu, exph, (double*)w, dst);
       SG_LAUNCHED();
