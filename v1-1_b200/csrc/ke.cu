@@ -35,8 +35,8 @@ struct KeArgs {
 };
 
 // pass 1: xy planes
-__global__ void __launch_bounds__(256) ke_xy_kernel(const double2* __restrict__ in,
-                                                    double2* __restrict__ out, KeArgs ka) {
+__global__ void __launch_bounds__(256) ke_xy_kernel(const double2* in,
+                                                    double2* out, KeArgs ka) {
   extern __shared__ double sm[];
   const int N = ka.N, S = ka.S, n8 = ka.n8;
   double* Ks = sm;             // n8 x S
@@ -44,6 +44,8 @@ __global__ void __launch_bounds__(256) ke_xy_kernel(const double2* __restrict__ 
   double* Xi = Xr + n8 * S;    // n8 x S
   const int z = blockIdx.x, orb = blockIdx.y;
   const double2* src = in + (long long)orb * ka.G + (long long)z * N * N;
+  grid_dependency_wait();
+  grid_dependents_launch();
   // staged in batches of 8 elements per thread: all 8 loads are in flight before
   // the first shared-memory store
   for (int i0 = threadIdx.x; i0 < n8 * S; i0 += 8 * blockDim.x) {
@@ -105,8 +107,8 @@ __global__ void __launch_bounds__(256) ke_xy_kernel(const double2* __restrict__ 
 }
 
 // pass 2: xz planes, O'[z][x] = sum_l K[z][l] X'[l][x], added into out
-__global__ void __launch_bounds__(256) ke_z_kernel(const double2* __restrict__ in,
-                                                   double2* __restrict__ out, KeArgs ka) {
+__global__ void __launch_bounds__(256) ke_z_kernel(const double2* in,
+                                                   double2* out, KeArgs ka) {
   extern __shared__ double sm[];
   const int N = ka.N, S = ka.S, n8 = ka.n8;
   double* Ks = sm;
@@ -115,6 +117,8 @@ __global__ void __launch_bounds__(256) ke_z_kernel(const double2* __restrict__ i
   const int y = blockIdx.x, orb = blockIdx.y;
   const long long NN = (long long)N * N;
   const double2* src = in + (long long)orb * ka.G + (long long)y * N;
+  grid_dependency_wait();
+  grid_dependents_launch();
   for (int i0 = threadIdx.x; i0 < n8 * S; i0 += 8 * blockDim.x) {
     double kv[8];
     double2 xv[8];
@@ -202,13 +206,10 @@ int mult_ke(Ctx& c, const double2* in, double2* out, int howmany, bool extra, do
   SG_CUDA(attr);
   {
     ProfScope ps(c, ST_KE_XY);
-    ke_xy_kernel<<<dim3(N, howmany), 256, smem, c.stream>>>(in, out, ka);
-    SG_LAUNCHED();
+    SG_TRY(launch_early(c.stream, ke_xy_kernel, dim3(N, howmany), dim3(256), smem, in, out, ka));
   }
   ProfScope ps(c, ST_KE_Z);
-  ke_z_kernel<<<dim3(N, howmany), 256, smem, c.stream>>>(in, out, ka);
-  SG_LAUNCHED();
-  return SINCGPU_OK;
+  return launch_early(c.stream, ke_z_kernel, dim3(N, howmany), dim3(256), smem, in, out, ka);
 }
 
 }  // namespace sincgpu

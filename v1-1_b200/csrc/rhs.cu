@@ -38,14 +38,16 @@ constexpr int kRhsSmemMax = 64 * 1024;
 constexpr int LMT = 2;            // fragments of 8 points per warp
 constexpr int kLinWarps = 8;
 template <int NS, int NT>
-__global__ void __launch_bounds__(32 * kLinWarps) lin_kernel(const double2* __restrict__ base,
-                                                             const double2* __restrict__ src0,
-                                                             const double2* __restrict__ mat0,
-                                                             const double2* __restrict__ src1,
-                                                             const double2* __restrict__ mat1, double sgn, int n,
-                                                             long long G, double2* __restrict__ out) {
+__global__ void __launch_bounds__(32 * kLinWarps) lin_kernel(const double2* base,
+                                                             const double2* src0,
+                                                             const double2* mat0,
+                                                             const double2* src1,
+                                                             const double2* mat1, double sgn, int n,
+                                                             long long G, double2* out) {
   constexpr int KS = 2 * NT;  // K steps of 4 = 2 orbitals
   extern __shared__ double lsm[];  // [NS][KS][NT][32]
+  grid_dependency_wait();
+  grid_dependents_launch();
   const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
   for (int e = tid; e < NS * KS * NT * 32; e += blockDim.x) {
     const int l = e & 31, nt = (e >> 5) % NT, ks = (e >> 5) / NT % KS, s = (e >> 5) / (NT * KS);
@@ -105,13 +107,15 @@ __global__ void __launch_bounds__(32 * kLinWarps) lin_kernel(const double2* __re
 
 // s_i = acc(x,i) + sum_k V(x,k,i) phi_k(x) over i in [i0, i0+ni); then, when
 // `dentime`, t_i = timefac * sum_j s_j inv(j,i) (all n orbitals present).
-__global__ void __launch_bounds__(TXO * kMaxOrbRhs) redpot_kernel(const double2* __restrict__ phi,
-                                                           const double2* __restrict__ V,
-                                                           const double2* __restrict__ acc_in,
-                                                           const double2* __restrict__ inv, double2 timefac,
+__global__ void __launch_bounds__(TXO * kMaxOrbRhs) redpot_kernel(const double2* phi,
+                                                           const double2* V,
+                                                           const double2* acc_in,
+                                                           const double2* inv, double2 timefac,
                                                            int n, int i0, int ni, int dentime, long long G,
-                                                           double2* __restrict__ out) {
+                                                           double2* out) {
   extern __shared__ double2 rsm[];
+  grid_dependency_wait();
+  grid_dependents_launch();
   double2* sinv = rsm;                 // n*n (dentime)
   double2* sph = rsm + n * n;          // n x TXO
   double2* ss = sph + n * TXO;         // n x TXO (dentime)
@@ -250,9 +254,11 @@ __global__ void __launch_bounds__(TXO * kMaxOrbRhs) blendq_build_kernel(
 
 // out(x,i) = timefac (sum_j Y(x,j) M(j,i) + sum_k Q(x,k,i) xin(x,k))
 __global__ void __launch_bounds__(TXO * kMaxOrbRhs) blendq_apply_kernel(
-    const double2* __restrict__ xin, const double2* __restrict__ Y, const double2* __restrict__ Q,
-    const double2* __restrict__ M, double2 timefac, int n, long long G, double2* __restrict__ out) {
+    const double2* xin, const double2* Y, const double2* Q,
+    const double2* M, double2 timefac, int n, long long G, double2* out) {
   extern __shared__ double2 rsm[];
+  grid_dependency_wait();
+  grid_dependents_launch();
   double2* sM = rsm;            // n*n
   double2* sx = sM + n * n;     // n x TXO
   double2* sy = sx + n * TXO;   // n x TXO
@@ -360,14 +366,16 @@ __global__ void __launch_bounds__(128) dots_reduce_kernel(const double2* __restr
 constexpr int kDotWarps = 16, kDotBlocks = 148;
 constexpr int dot_points(int nt) { return nt <= 3 ? 16 : 8; }  // points per step of a warp (by registers)
 template <int NT>
-__global__ void __launch_bounds__(32 * kDotWarps) dots_mma_kernel(const double2* __restrict__ P,
-                                                                  const double2* __restrict__ T,
-                                                                  const double2* __restrict__ X,
-                                                                  const double2* __restrict__ O, int n, long long G,
-                                                                  double2* __restrict__ part, double2* __restrict__ D,
-                                                                  unsigned* __restrict__ count) {
+__global__ void __launch_bounds__(32 * kDotWarps) dots_mma_kernel(const double2* P,
+                                                                  const double2* T,
+                                                                  const double2* X,
+                                                                  const double2* O, int n, long long G,
+                                                                  double2* part, double2* D,
+                                                                  unsigned* count) {
   extern __shared__ double dsm[];  // [kDotWarps][NT * NT * 64]
   __shared__ unsigned last;
+  grid_dependency_wait();
+  grid_dependents_launch();
   constexpr int NE = NT * NT * 64, kDotPts = dot_points(NT);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const long long W = (long long)gridDim.x * kDotWarps, w = (long long)warp * gridDim.x + blockIdx.x;
@@ -499,10 +507,8 @@ int launch_lin_t(Ctx& c, const double2* base, const double2* s0, const double2* 
   static const cudaError_t attr =
       cudaFuncSetAttribute(lin_kernel<NS, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   SG_CUDA(attr);
-  lin_kernel<NS, NT><<<ceil_div(c.G, 8 * LMT * kLinWarps), 32 * kLinWarps, sm, c.stream>>>(base, s0, m0, s1, m1, sgn,
-                                                                                          c.nspf, c.G, out);
-  SG_LAUNCHED();
-  return SINCGPU_OK;
+  return launch_early(c.stream, lin_kernel<NS, NT>, dim3(ceil_div(c.G, 8 * LMT * kLinWarps)), dim3(32 * kLinWarps), sm,
+                      base, s0, m0, s1, m1, sgn, c.nspf, c.G, out);
 }
 
 // out = [base] + sgn (s0 m0 [+ s1 m1]) over the orbitals (lin_kernel)
@@ -534,9 +540,8 @@ int launch_dots_mma(Ctx& c, const double2* P, const double2* T, const double2* X
       cudaFuncSetAttribute(dots_mma_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   SG_CUDA(attr);
   const int nb = (int)std::min<long long>(kDotBlocks, ceil_div(c.G, dot_points(NT)));
-  dots_mma_kernel<NT><<<nb, 32 * kDotWarps, sm, c.stream>>>(P, T, X, O, c.nspf, c.G, part, D, c.d_count);
-  SG_LAUNCHED();
-  return SINCGPU_OK;
+  return launch_early(c.stream, dots_mma_kernel<NT>, dim3(nb), dim3(32 * kDotWarps), sm, P, T, X, O, c.nspf, c.G, part, D,
+                      c.d_count);
 }
 
 // one warp per orbital (n <= 32): every warp of a block has the same share of
@@ -612,10 +617,8 @@ int mult_reducedpot_range(Ctx& c, const double2* phi, const double2* redpot, int
   SG_CHECK(n <= kMaxOrbRhs, SINCGPU_ERANGE, "at most %d orbitals", kMaxOrbRhs);
   SG_TRY(rhs_attrs());
   ProfScope ps(c, ST_RHS_REDPOT);
-  redpot_kernel<<<ceil_div(c.G, TXO), tile_for(n), smem_redpot(n), c.stream>>>(
-      phi, redpot, nullptr, nullptr, make_double2(1, 0), n, i0, ni, 0, c.G, out);
-  SG_LAUNCHED();
-  return SINCGPU_OK;
+  return launch_early(c.stream, redpot_kernel, dim3(ceil_div(c.G, TXO)), tile_for(n), smem_redpot(n), phi, redpot, nullptr,
+                      nullptr, make_double2(1, 0), n, i0, ni, 0, c.G, out);
 }
 
 int mult_reducedpot(Ctx& c, const double2* phi, const double2* redpot, double2* out) {
@@ -728,10 +731,8 @@ int actreduced_blendq(Ctx& c, const double2* x, double2 timefac, double zfield, 
   SG_CHECK(Q, SINCGPU_ESTATE, "blended reduced potential not prepared");
   SG_TRY(mult_ke(c, x, t.Y, n, true, zfield));
   ProfScope ps(c, ST_RHS_REDPOT);
-  blendq_apply_kernel<<<ceil_div(c.G, TXO), tile_for(n), smem_bq_apply(n), c.stream>>>(
-      x, t.Y, Q, Q + (size_t)c.G * n * n, timefac, n, c.G, out);
-  SG_LAUNCHED();
-  return SINCGPU_OK;
+  return launch_early(c.stream, blendq_apply_kernel, dim3(ceil_div(c.G, TXO)), tile_for(n), smem_bq_apply(n), x, t.Y, Q,
+                      Q + (size_t)c.G * n * n, timefac, n, c.G, out);
 }
 
 int actreduced_temps(Ctx& c, double2** S, double2** T) {
@@ -754,9 +755,8 @@ int actreduced_post(Ctx& c, const double2* phi, const double2* proj, const doubl
   double2* dst = projflag == 1 ? T : out;
   if (!t_ready) {
     ProfScope ps(c, ST_RHS_REDPOT);
-    redpot_kernel<<<bt, tile_for(n), smem_redpot(n), c.stream>>>(phi, redpot, S, invdenmat, timefac, n, 0, n,
-                                                           dentimeflag ? 1 : 0, G, dst);
-    SG_LAUNCHED();
+    SG_TRY(launch_early(c.stream, redpot_kernel, dim3(bt), tile_for(n), smem_redpot(n), phi, redpot, S, invdenmat, timefac,
+                        n, 0, n, dentimeflag ? 1 : 0, G, dst));
   }
   if (projflag == 1) {
     ProfScope ps(c, ST_RHS_PROJ);
