@@ -220,9 +220,11 @@ __device__ __forceinline__ double2 warp_sum(double2 v) {
 template <bool DEN>
 __global__ void __launch_bounds__(128) rdm_gather_kernel(const long long* __restrict__ off,
                                                          const int2* __restrict__ ent,
-                                                         const double2* __restrict__ a1,
-                                                         const double2* __restrict__ a2, long long nel,
+                                                         const double2* a1,
+                                                         const double2* a2, long long nel,
                                                          double2* __restrict__ out) {
+  grid_dependency_wait();
+  grid_dependents_launch();
   const long long e = blockIdx.x * 4LL + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (e >= nel) return;
@@ -247,9 +249,11 @@ __global__ void __launch_bounds__(128) rdm_gather_kernel(const long long* __rest
 // singular value is far above the regularisation threshold the SVD formula is
 // the plain inverse, and sigma_min >= 1/||A^-1||_F certifies that; need_svd is
 // set otherwise.
-__global__ void __launch_bounds__(256) inverse_gj_kernel(const double2* __restrict__ A_in, int n,
+__global__ void __launch_bounds__(256) inverse_gj_kernel(const double2* A_in, int n,
                                                          double safe_sigma, double2* __restrict__ inv,
                                                          int* __restrict__ need_svd) {
+  grid_dependency_wait();
+  grid_dependents_launch();
   __shared__ double2 M[32][65];
   __shared__ double2 fcol[32];
   __shared__ int piv, sing;
@@ -323,9 +327,11 @@ __global__ void __launch_bounds__(256) inverse_gj_kernel(const double2* __restri
 // Regularised inverse of an n x n complex matrix by one-sided (Hestenes) Jacobi
 // SVD: A = U S V^H, inv = V f(S) U^H with f(s) = 1/s, 1/tol below tol, 0 at 0.
 // One warp, lane k owns row k.  Skipped when `need_svd` is 0.
-__global__ void __launch_bounds__(32) invmatsmooth_kernel(const double2* __restrict__ A_in, int n,
+__global__ void __launch_bounds__(32) invmatsmooth_kernel(const double2* A_in, int n,
                                                           double tol, double2* __restrict__ inv,
-                                                          const int* __restrict__ need_svd) {
+                                                          const int* need_svd) {
+  grid_dependency_wait();
+  grid_dependents_launch();
   if (need_svd && *need_svd == 0) return;
   __shared__ double2 A[32 * 32], V[32 * 32];
   __shared__ double sv[32];
@@ -353,17 +359,16 @@ int ci_denmat(Ctx& c, const double2* avec, double2* denmat, double2* invdenmat, 
   SG_CHECK(s.attached, SINCGPU_ESTATE, "no walk tables attached");
   const int n = c.nspf;
   ProfScope ps(c, ST_CI);
-  rdm_gather_kernel<true><<<ceil_div((long long)n * n, 4), 128, 0, c.stream>>>(s.den_off, s.den_ent, avec,
-                                                                              avec, (long long)n * n, denmat);
-  SG_LAUNCHED();
+  const bool early = early_evaluation(c.G);
+  SG_TRY(launch_waiting(c.stream, early, rdm_gather_kernel<true>, dim3(ceil_div((long long)n * n, 4)), dim3(128), 0, s.den_off,
+                        s.den_ent, avec, avec, (long long)n * n, denmat));
   if (invdenmat) {
     SG_TRY(c.ws_ci2.ensure(sizeof(double2) * n * n + 256));
     int* flag = (int*)((char*)c.ws_ci2.ptr + sizeof(double2) * n * n);
     // plain inverse is the SVD formula when sigma_min >= 1e-6 >> denreg
-    inverse_gj_kernel<<<1, 256, 0, c.stream>>>(denmat, n, std::max(1e-6, 1e4 * denreg), invdenmat, flag);
-    SG_LAUNCHED();
-    invmatsmooth_kernel<<<1, 32, 0, c.stream>>>(denmat, n, denreg, invdenmat, flag);
-    SG_LAUNCHED();
+    SG_TRY(launch_waiting(c.stream, early, inverse_gj_kernel, dim3(1), dim3(256), 0, denmat, n, std::max(1e-6, 1e4 * denreg),
+                        invdenmat, flag));
+    SG_TRY(launch_waiting(c.stream, early, invmatsmooth_kernel, dim3(1), dim3(32), 0, denmat, n, denreg, invdenmat, flag));
   }
   return SINCGPU_OK;
 }
@@ -373,9 +378,8 @@ int ci_tally(Ctx& c, const double2* a1, const double2* a2, double2* tally) {
   SG_CHECK(s.attached, SINCGPU_ESTATE, "no walk tables attached");
   const long long n4 = (long long)c.nspf * c.nspf * c.nspf * c.nspf;
   ProfScope ps(c, ST_CI);
-  rdm_gather_kernel<false><<<ceil_div(n4, 4), 128, 0, c.stream>>>(s.tal_off, s.tal_ent, a1, a2, n4, tally);
-  SG_LAUNCHED();
-  return SINCGPU_OK;
+  return launch_waiting(c.stream, early_evaluation(c.G), rdm_gather_kernel<false>, dim3(ceil_div(n4, 4)), dim3(128), 0,
+                        s.tal_off, s.tal_ent, a1, a2, n4, tally);
 }
 
 // ---------------------------------------------------------------------------
@@ -705,20 +709,9 @@ static int launch_sigma(Ctx& c, bool early, const double2* xpot, const double2* 
     return SINCGPU_OK;
   }
   const bool four = s.nc <= kSigmaWarps / 4;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ceil_div(s.nc, four ? 1 : 4), 1, 1);
-  cfg.blockDim = dim3(128, 1, 1);
-  cfg.stream = c.stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = early ? 1 : 0;
-  SG_CUDA(cudaLaunchKernelEx(&cfg, four ? sigma_small_kernel<4> : sigma_small_kernel<1>, (const long long*)s.dhop_off,
-                             (const int*)s.dhop, xpot, (const long long*)s.shop_off, (const int*)s.shop, xone,
-                             (const double2*)s.xz, ez, diag, in, s.nc, out, tf, scaled ? 1 : 0, skip));
-  count_launch();
-  return SINCGPU_OK;
+  return launch_waiting(c.stream, early, four ? sigma_small_kernel<4> : sigma_small_kernel<1>,
+                        dim3(ceil_div(s.nc, four ? 1 : 4)), dim3(128), 0, s.dhop_off, s.dhop, xpot, s.shop_off, s.shop,
+                        xone, s.xz, ez, diag, in, s.nc, out, tf, scaled ? 1 : 0, skip);
 }
 
 // z-dipole expectation (dipolesub_one, MCTDH.SRC/dipolesub.f90:20-125, z part):

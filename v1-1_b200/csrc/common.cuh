@@ -61,10 +61,11 @@ __host__ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // the kernel behind may start once every CTA has come here
 __device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;"); }
-// Launch of a kernel that begins with the wait: its CTAs may be in place before the kernel in
-// front has ended, which takes 1 to 1.5 us off every boundary of a chain.
+// Launch of a kernel that begins with the wait.  `early`: its CTAs may be in place before the
+// kernel in front has ended, which takes 1 to 1.5 us off a boundary of a chain.
 template <class... KA, class... A>
-static int launch_early(cudaStream_t stream, void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, A... args) {
+static int launch_waiting(cudaStream_t stream, bool early, void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem,
+                          A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -74,11 +75,19 @@ static int launch_early(cudaStream_t stream, void (*kernel)(KA...), dim3 grid, d
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = early ? 1 : 0;
   SG_CUDA(cudaLaunchKernelEx(&cfg, kernel, (KA)args...));
   count_launch();
   return SINCGPU_OK;
 }
+template <class... KA, class... A>
+static int launch_early(cudaStream_t stream, void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, A... args) {
+  return launch_waiting(stream, true, kernel, grid, block, smem, args...);
+}
+// The two streams of a mean-field evaluation: early at the grids where the boundaries count
+// (21^3 / 5 orbitals: 65 -> 57 us).  On larger ones the waiting CTAs of one stream take the
+// room that the other's kernels would use (57^3 / 11: 1.95 -> 2.01 ms, 41^3 / 10: 565 -> 570 us).
+__host__ __device__ constexpr bool early_evaluation(long long points) { return points <= 32768; }
 // acc += v*m with explicit FMAs (one rounding order wherever it is used)
 __device__ __forceinline__ void cfma(double2& acc, double2 v, double2 m) {
   acc.x = fma(v.x, m.x, fma(-v.y, m.y, acc.x));

@@ -543,8 +543,10 @@ static size_t twoe_patch_smem(int M, int n) {
 // splits g, g + 8, ...) in a fixed order and warp 0 adds the eight partial sums in
 // order.  Elements of the lower-triangle tiles (tile(m) > tile(n), never computed)
 // are read mirrored.
-__global__ void __launch_bounds__(256) split_reduce_kernel(const double* __restrict__ part, int nsplit, int M,
+__global__ void __launch_bounds__(256) split_reduce_kernel(const double* part, int nsplit, int M,
                                                            int TT, double* __restrict__ C) {
+  grid_dependency_wait();
+  grid_dependents_launch();
   __shared__ double acc[8][32];
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
   const long long MM = (long long)M * M;
@@ -570,9 +572,11 @@ __global__ void __launch_bounds__(256) split_reduce_kernel(const double* __restr
 // twoematel(a1,b1,a2,b2) from C = [[UR,US],[VR,VS]]
 // lut[a + n*b] = 2*p + conj  (hermitian pairs a<=b), or p for the general list.
 // rowof[p], rowof[npair + p]: the rows of C with pair p's real and imaginary part (-1: zero)
-__global__ void twoe_assemble_kernel(const double* __restrict__ C, const int* __restrict__ lut,
+__global__ void twoe_assemble_kernel(const double* C, const int* __restrict__ lut,
                                      const int* __restrict__ rowof, int M, int npair, int n, int herm,
                                      double2* __restrict__ out) {
+  grid_dependency_wait();
+  grid_dependents_launch();
   long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long n4 = (long long)n * n * n * n;
   if (idx >= n4) return;
@@ -781,13 +785,12 @@ int twoe_matel(Ctx& c, const double2* phi1, const double2* phi2, const int* h_pa
     SG_LAUNCHED();
   }
   ProfScope ps(c, ST_TWOE_FINISH);
-  split_reduce_kernel<<<ceil_div(MM, 32), 256, 0, c.stream>>>(part, nsplit, M, TT, C);
-  SG_LAUNCHED();
+  const bool early = early_evaluation(c.G);
+  SG_TRY(launch_waiting(c.stream, early, split_reduce_kernel, dim3(ceil_div(MM, 32)), dim3(256), 0, part, nsplit, M, TT,
+                        C));
   const long long n4 = (long long)n * n * n * n;
-  twoe_assemble_kernel<<<ceil_div(n4, 256), 256, 0, c.stream>>>(C, d_lut, d_rowof, M, npair, n, herm ? 1 : 0,
-                                                                 twoematel);
-  SG_LAUNCHED();
-  return SINCGPU_OK;
+  return launch_waiting(c.stream, early, twoe_assemble_kernel, dim3(ceil_div(n4, 256)), dim3(256), 0, C, d_lut, d_rowof, M,
+                        npair, n, herm ? 1 : 0, twoematel);
 }
 
 // ---------------------------------------------------------------------------
@@ -1082,14 +1085,16 @@ __global__ void __launch_bounds__(256, FN <= 7 ? 3 : 2) rp_dmma_kernel(const dou
 // HBM.  Dynamic shared memory: the K loop's stages, then the epilogue's tile.
 constexpr int RPV = DM + 2;  // tile row stride (doubles): conflict-free accumulator stores
 template <int FN>
-__global__ void __launch_bounds__(256, 3) rp_apply_kernel(const double* __restrict__ Rpl, const double* __restrict__ Wm,
+__global__ void __launch_bounds__(256, 3) rp_apply_kernel(const double* Rpl, const double* Wm,
                                                        const int* __restrict__ rows, int packed, int K, int NC,
                                                        long long G, double2* __restrict__ out,
                                                        const int* __restrict__ tmap, int n,
-                                                       const double2* __restrict__ phi,
-                                                       const double2* __restrict__ S,
-                                                       const double2* __restrict__ inv, double2 timefac,
+                                                       const double2* phi,
+                                                       const double2* S,
+                                                       const double2* inv, double2 timefac,
                                                        double2* __restrict__ T) {
+  grid_dependency_wait();
+  grid_dependents_launch();
   extern __shared__ __align__(16) double rp_sm[];
   auto As = reinterpret_cast<double (*)[DK][DAS]>(rp_sm);
   auto Bs = reinterpret_cast<double (*)[DK][16 * FN + 4]>(rp_sm + DST * DK * DAS);
@@ -1271,9 +1276,9 @@ static int reduced_pot_impl(Ctx& c, const double* Rpl, const int* h_pa, const in
       const size_t sm = rp_apply_smem(n, NC, fn);
 #define SG_RP_APPLY(FN)                                                                                  \
   case FN:                                                                                               \
-    rp_apply_kernel<FN><<<grid, 256, sm, c.stream>>>(Rpl, Wm, d_rows, packed ? 1 : 0, K, NC, c.G, reducedpot, \
-                                                     d_tmap, n, apply->phi, apply->S, apply->inv, apply->timefac,      \
-                                                     apply->T);                                            \
+    SG_TRY(launch_waiting(c.stream, early_evaluation(c.G), rp_apply_kernel<FN>, dim3(grid), dim3(256), sm, Rpl, Wm,     \
+                          d_rows, packed ? 1 : 0, K, NC, c.G, reducedpot, d_tmap, n, apply->phi, apply->S, apply->inv, \
+                          apply->timefac, apply->T));                                                      \
     break;
       switch (fn) {
         SG_RP_APPLY(2)
@@ -1285,7 +1290,6 @@ static int reduced_pot_impl(Ctx& c, const double* Rpl, const int* h_pa, const in
           SG_RP_APPLY(7)
       }
 #undef SG_RP_APPLY
-      SG_LAUNCHED();
       apply->done = true;
       return SINCGPU_OK;
     }

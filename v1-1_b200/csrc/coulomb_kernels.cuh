@@ -59,7 +59,9 @@ __device__ __forceinline__ void load_roots(C* roots, const C* g, int P) {
 // CX: rows of rho -> DFT along x -> W1
 template <int P1, int P2, bool DENS, class C>
 __global__ void __launch_bounds__((P1 > P2 ? P1 : P2) * lines_for(P1 * P2)) coul_fwd_x_t(
-    const double2* __restrict__ phi1, const double2* __restrict__ phi2, CoulArgs<C> ca) {
+    const double2* phi1, const double2* phi2, CoulArgs<C> ca) {
+  grid_dependency_wait();
+  grid_dependents_launch();
   constexpr int P = P1 * P2, S = P1 > P2 ? P1 : P2, TL = lines_for(P);
   __shared__ C roots[P];
   __shared__ C ex[(P + 1) * TL];
@@ -100,6 +102,8 @@ __global__ void __launch_bounds__((P1 > P2 ? P1 : P2) * lines_for(P1 * P2)) coul
 // CY: W1 columns (y < N) -> DFT along y -> W2
 template <int P1, int P2, class C>
 __global__ void __launch_bounds__((P1 > P2 ? P1 : P2) * lines_for(P1 * P2)) coul_fwd_y_t(CoulArgs<C> ca) {
+  grid_dependency_wait();
+  grid_dependents_launch();
   constexpr int P = P1 * P2, TL = lines_for(P);
   __shared__ C roots[P];
   __shared__ C ex[P * TL];
@@ -130,6 +134,8 @@ __global__ void __launch_bounds__((P1 > P2 ? P1 : P2) * lines_for(P1 * P2)) coul
 // three with spilled registers measured slower, 4.8 -> 5.9 ms per evaluation.)
 template <int P1, int P2, class C>
 __global__ void __launch_bounds__((P1 > P2 ? P1 : P2) * lines_for_z<C>(P1 * P2)) coul_z_t(CoulArgs<C> ca) {
+  grid_dependency_wait();
+  grid_dependents_launch();
   constexpr int P = P1 * P2, TL = lines_for_z<C>(P);
   __shared__ C roots[P];
   __shared__ C ex[P * TL];
@@ -376,6 +382,8 @@ __global__ void __launch_bounds__((P1 > P2 ? P1 : P2) * lines_for_ztma<C>(P1 * P
 // CYI: W2 columns along ky (all P) -> inverse DFT -> W1 (y < N)
 template <int P1, int P2, class C>
 __global__ void __launch_bounds__((P1 > P2 ? P1 : P2) * lines_for(P1 * P2)) coul_inv_y_t(CoulArgs<C> ca) {
+  grid_dependency_wait();
+  grid_dependents_launch();
   constexpr int P = P1 * P2, TL = lines_for(P);
   __shared__ C roots[P];
   __shared__ C ex[P * TL];
@@ -406,6 +414,8 @@ __global__ void __launch_bounds__((P1 > P2 ? P1 : P2) * lines_for(P1 * P2)) coul
 template <int P1, int P2, bool DENS, class C>
 __global__ void __launch_bounds__((P1 > P2 ? P1 : P2) * lines_for(P1 * P2)) coul_inv_x_t(
     CoulArgs<C> ca, double* __restrict__ Rpl, double2* __restrict__ full, int herm) {
+  grid_dependency_wait();
+  grid_dependents_launch();
   constexpr int P = P1 * P2, S = P1 > P2 ? P1 : P2, TL = lines_for(P);
   __shared__ C roots[P];
   __shared__ C ex[(P + 1) * TL];
@@ -502,18 +512,15 @@ int coul_launch(Ctx& c, const CoulArgs<C>& ca, int np, bool dens, const double2*
     }
     return SINCGPU_OK;
   }
+  const bool early = early_evaluation(c.G);
   {
     ProfScope ps(c, ST_COUL_FWD_X);
-    if (dens)
-      coul_fwd_x_t<P1, P2, true, C><<<dim3(np, nrow), nthr, 0, c.stream>>>(src1, nullptr, ca);
-    else
-      coul_fwd_x_t<P1, P2, false, C><<<dim3(np, nrow), nthr, 0, c.stream>>>(src1, src2, ca);
-    SG_LAUNCHED();
+    SG_TRY(launch_waiting(c.stream, early, dens ? coul_fwd_x_t<P1, P2, true, C> : coul_fwd_x_t<P1, P2, false, C>,
+                          dim3(np, nrow), dim3(nthr), 0, src1, dens ? nullptr : src2, ca));
   }
   {
     ProfScope ps(c, ST_COUL_FWD_Y);
-    coul_fwd_y_t<P1, P2, C><<<dim3(ncol, 1, np), nthr, 0, c.stream>>>(ca);
-    SG_LAUNCHED();
+    SG_TRY(launch_waiting(c.stream, early, coul_fwd_y_t<P1, P2, C>, dim3(ncol, 1, np), dim3(nthr), 0, ca));
   }
   {
     ProfScope ps(c, ST_COUL_Z);
@@ -538,6 +545,7 @@ int coul_launch(Ctx& c, const CoulArgs<C>& ca, int np, bool dens, const double2*
       const int ntf = ceil_div(P * P, TLT), ntiles = ntf * np;
       const int grid = std::min(ntiles, nsm * occ);
       coul_z_tma_t<P1, P2, C><<<grid, S * TLT, dyn, c.stream>>>(ca, *zmap, ntf, ntiles, slab_stride, err);
+      SG_LAUNCHED();
     } else if constexpr (P1 == 2 * P2 && P > 128) {
       // (the paired pass reads the whole real spectrum table, built above 128)
       if (c.coul_z2) {
@@ -547,26 +555,22 @@ int coul_launch(Ctx& c, const CoulArgs<C>& ca, int np, bool dens, const double2*
             coul_z2_t<P1, P2, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
         SG_CUDA(attr);
         coul_z2_t<P1, P2, C><<<dim3(ceil_div(P * P, TL2), 1, np), P2 * TL2, dyn, c.stream>>>(ca);
+        SG_LAUNCHED();
       } else {
-        coul_z_t<P1, P2, C><<<dim3(nzc, 1, np), S * TLZ, 0, c.stream>>>(ca);
+        SG_TRY(launch_waiting(c.stream, early, coul_z_t<P1, P2, C>, dim3(nzc, 1, np), dim3(S * TLZ), 0, ca));
       }
     } else {
-      coul_z_t<P1, P2, C><<<dim3(nzc, 1, np), S * TLZ, 0, c.stream>>>(ca);
+      SG_TRY(launch_waiting(c.stream, early, coul_z_t<P1, P2, C>, dim3(nzc, 1, np), dim3(S * TLZ), 0, ca));
     }
-    SG_LAUNCHED();
   }
   {
     ProfScope ps(c, ST_COUL_INV_Y);
-    coul_inv_y_t<P1, P2, C><<<dim3(ncol, 1, np), nthr, 0, c.stream>>>(ca);
-    SG_LAUNCHED();
+    SG_TRY(launch_waiting(c.stream, early, coul_inv_y_t<P1, P2, C>, dim3(ncol, 1, np), dim3(nthr), 0, ca));
   }
   {
     ProfScope ps(c, ST_COUL_INV_X);
-    if (dens)
-      coul_inv_x_t<P1, P2, true, C><<<dim3(nrow, 1, np), nthr, 0, c.stream>>>(ca, Rpl, full, 0);
-    else
-      coul_inv_x_t<P1, P2, false, C><<<dim3(nrow, 1, np), nthr, 0, c.stream>>>(ca, Rpl, full, herm ? 1 : 0);
-    SG_LAUNCHED();
+    SG_TRY(launch_waiting(c.stream, early, dens ? coul_inv_x_t<P1, P2, true, C> : coul_inv_x_t<P1, P2, false, C>,
+                          dim3(nrow, 1, np), dim3(nthr), 0, ca, Rpl, full, !dens && herm ? 1 : 0));
   }
   return SINCGPU_OK;
 }
