@@ -80,7 +80,7 @@ int sincgpu_fft_length(sincgpu_ctx* ctx);
  * faster at every measured length once whole pair lists go in one launch);
  * "twoe_tile" (twoematel tile edge 16R: 0 = least padding, 2..9 = R);
  * "orth_onepass" (1, default: the coefficients of an orbital Arnoldi step's
- * orthogonalisation come from one pass of dots, three launches a step; 0: one
+ * orthogonalisation come from one pass of dots; 0: one
  * projection after another, as "orth_fused" says; results agree to rounding);
  * "orth_fused" (with orth_onepass 0, 1: the orbital Arnoldi orthogonalisation of one
  * Krylov step in one cooperative launch with bounded grid barriers, 0: one launch per
@@ -102,9 +102,9 @@ int sincgpu_fft_length(sincgpu_ctx* ctx);
  * a copy stream, and the Coulomb pair loop starts on the pairs of the first
  * group while the others are in flight; 1: one copy before the evaluation;
  * bitwise the same); "kry_cluster" (1, default: the A-vector Krylov's
- * Gram-Schmidt step and update run on a cluster of 8 CTAs, its coefficients from one
+ * Gram-Schmidt step and update run on a cluster of 16 CTAs, its coefficients from one
  * pass of dot products summed through distributed shared memory, for vectors of up to
- * 112640 reals; 0: one CTA, one projection after another; results agree to rounding); "orb_blendq" (1, default: an orbital Krylov
+ * 129600 reals; 0: one CTA, one projection after another; results agree to rounding); "orb_blendq" (1, default: an orbital Krylov
  * call with two mean-field slots folds their reduced potentials and density
  * matrices into one blended potential once, and each Jacobian product reads
  * that; 0: each product reads both slots; results agree to rounding);

@@ -217,7 +217,7 @@ struct Ctx {
   int twoe_symdiag = 0;   // 1: multi-tile twoematel computes its diagonal tiles' lower blocks only
   int twoe_tile = 0;      // twoematel tile edge 16R: 0 = least padding, 2..9 = that R
   int orth_fused = 1;     // 1: an orbital Arnoldi step's orthogonalisation in one cooperative launch
-  int orth_onepass = 1;   // 1: the orbital Arnoldi coefficients from one pass of dots, three launches a step
+  int orth_onepass = 1;   // 1: the orbital Arnoldi coefficients from one pass of dots
   int kry_cluster = 1;    // 1: A-vector Gram-Schmidt and update on a cluster of CTAs (0: one CTA)
   int orb_blendq = 1;     // 1: the orbital Jacobian reads one blended reduced potential (0: both slots')
   int rhs_overlap = 1;    // 1: the fused orbital-RHS entry runs its CI part and the mix + kinetic
