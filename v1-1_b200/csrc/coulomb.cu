@@ -322,8 +322,11 @@ static int coulomb_dens_scratch_t(Ctx& c, const double2* dens, int m, double2* r
   SG_CHECK(per_dens <= scratch_bytes, SINCGPU_ERANGE,
            "one density on a %d^3 grid (FFT length %d) needs %zu bytes of scratch; the fixed "
            "scratch holds %zu bytes", N, P, per_dens, scratch_bytes);
-  if (use_half(c)) {  // less than the five passes need, or (N <= 21) far less than the scratch
+  if (use_half(c)) {  // less than the five passes need with every plan of coul_half.h
     const size_t per = (size_t)half_pair_bytes(c);
+    SG_CHECK(per <= scratch_bytes, SINCGPU_ERANGE,
+             "one density on a %d^3 grid (half-length %d) needs %zu bytes of scratch; the fixed scratch holds %zu bytes",
+             N, c.hM, per, scratch_bytes);
     const int chunk = (int)std::min<size_t>({scratch_bytes / per, (size_t)m, 65535});
     HalfArgs ha = half_args(c, scratch, chunk, m, false);
     for (int p0 = 0; p0 < m; p0 += chunk) {
