@@ -80,11 +80,12 @@ int sincgpu_fft_length(sincgpu_ctx* ctx);
  * faster at every measured length once whole pair lists go in one launch);
  * "twoe_tile" (twoematel tile edge 16R: 0 = least padding, 2..9 = R);
  * "orth_onepass" (1, default: the coefficients of an orbital Arnoldi step's
- * orthogonalisation come from one pass of dots; 0: one
- * projection after another, as "orth_fused" says; results agree to rounding);
- * "orth_fused" (with orth_onepass 0, 1: the orbital Arnoldi orthogonalisation of one
- * Krylov step in one cooperative launch with bounded grid barriers, 0: one launch per
- * dot, projection and norm; the results are bitwise the same); "rhs_overlap" (1: the
+ * orthogonalisation come from one pass of dots; 0: one projection after another;
+ * results agree to rounding);
+ * "orth_fused" (1, default: that orthogonalisation in one cooperative launch with
+ * bounded grid barriers where the vector fits its registers; 0: separate launches, three
+ * with orth_onepass, else one per dot, projection and norm; the results are bitwise the
+ * same); "rhs_overlap" (1: the
  * A-vector orbital-RHS entry runs the RDMs, the density-matrix inverse and the
  * kinetic contraction on a second stream of the context beside the Coulomb
  * passes, then twoematel there beside reducedpot and the apply, joined by

@@ -278,6 +278,7 @@ __global__ void __launch_bounds__(kLvThreads, 2) lv_arnoldi_orth_kernel(const do
 // sides; where p fits the registers, lv_orth_onepass_kernel does these three passes in
 // one launch with two barriers: 48 -> 35 us a step at 41^3 / 10 orbitals, ten vectors
 // (cold caches; three launches took 47).
+// The same grid, element assignment, partial sums and orders in both forms, so the same bits.
 constexpr int kRows = 8;
 
 // adds this CTA to *count; true in the last one (which resets it for the next launch)
@@ -500,13 +501,18 @@ __global__ void __launch_bounds__(kLvThreads, 2) lv_project_kernel(const double2
   double s = 0.0;
   for (long long k = blockIdx.x * (long long)kLvThreads + tid; k < nv; k += (long long)gridDim.x * kLvThreads) {
     double2 x = p[k];
-    for (int c0 = 0; c0 <= j; c0 += kRows) {
+    // fours of rows from the last to the first, two fours in registers at a time
+    for (int c0 = j / 4 * 4; c0 >= 0; c0 -= kRows) {
       double2 v[kRows];
 #pragma unroll
-      for (int q = 0; q < kRows; ++q) v[q] = c0 + q <= j ? V[(long long)(c0 + q) * nv + k] : make_double2(0.0, 0.0);
+      for (int q = 0; q < kRows; ++q) {
+        const int i = c0 + q - (q < 4 ? 0 : kRows);
+        v[q] = i >= 0 && i <= j ? V[(long long)i * nv + k] : make_double2(0.0, 0.0);
+      }
 #pragma unroll
       for (int q = 0; q < kRows; ++q) {
-        const double c = c0 + q <= j ? h[c0 + q] : 0.0;
+        const int i = c0 + q - (q < 4 ? 0 : kRows);
+        const double c = i >= 0 && i <= j ? h[i] : 0.0;
         x.x = fma(-c, v[q].x, x.x);
         x.y = fma(-c, v[q].y, x.y);
       }
@@ -845,8 +851,8 @@ int expospfprop(Ctx& c, double2* phi, const MeanFieldSlot* slots, double tin, do
   bool w_zero = true;
   SG_CUDA(cudaMemsetAsync(o.w, 0, sizeof(double2) * nv, c.stream));
   const int lvg = kLvBlocks;
-  const bool one_launch = nv <= (long long)kOrthE * lvg * kLvThreads && orth_fits();
-  const bool orth_fused = c.orth_fused && one_launch;
+  // one cooperative launch per Arnoldi step, where it is allowed and p fits the registers
+  const bool one_launch = c.orth_fused && nv <= (long long)kOrthE * lvg * kLvThreads && orth_fits();
   SG_CUDA(cudaMemsetAsync(o.gbar, 0, 3 * sizeof(unsigned), c.stream));
   SG_CUDA(cudaMemsetAsync(o.st, 0, sizeof(OrbKryState), c.stream));
   const int ub = std::min<long long>(ceil_div(nv, 256), 148 * 8);
@@ -909,7 +915,7 @@ int expospfprop(Ctx& c, double2* phi, const MeanFieldSlot* slots, double tin, do
         SG_LAUNCHED();
         lv_scale_kernel<<<lvg, kLvThreads, 0, c.stream>>>(p, nv, o.st);
         SG_LAUNCHED();
-      } else if (orth_fused) {
+      } else if (one_launch) {
         const double2* Vc = o.V;
         double *P0 = o.part0, *P1 = o.part1, *H = o.Hm;
         OrbKryState* S = o.st;
