@@ -534,9 +534,14 @@ int ci_assemble(Ctx& c, const double2* twoematel, const double2* mats) {
   return SINCGPU_OK;
 }
 
+// a matrix element or target: read past the caches (`STREAM`) or kept in them
+template <bool STREAM, class T>
+__device__ __forceinline__ T load_hop(const T* p) {
+  return STREAM ? __ldcs(p) : __ldg(p);
+}
 // sum over [b, e) of m[h] a[hop[h]] by one warp's lanes (h = b + lane, + 32, ...), lane sums
 // in ascending h; the loads of U strides are in flight together
-template <int U, class MAT>
+template <int U, bool STREAM, class MAT>
 __device__ __forceinline__ double2 hop_sum(long long b, long long e, const int* __restrict__ hop, const MAT& mat,
                                            const double2* __restrict__ a) {
   double2 acc = make_double2(0.0, 0.0);
@@ -546,7 +551,7 @@ __device__ __forceinline__ double2 hop_sum(long long b, long long e, const int* 
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const bool ok = h + 32 * u < e;
-      t[u] = ok ? __ldcs(hop + h + 32 * u) : -1;
+      t[u] = ok ? load_hop<STREAM>(hop + h + 32 * u) : -1;
       m[u] = ok ? mat(h + 32 * u) : make_double2(0.0, 0.0);
     }
 #pragma unroll
@@ -558,47 +563,60 @@ __device__ __forceinline__ double2 hop_sum(long long b, long long e, const int* 
   return acc;
 }
 
-// sigma(c1) = const A(c1) + sum_dhops xpot A(dhop) + sum_shops (xone + ez xz) A(shop) + ez nucdip A(c1),
-// times `tf` when `scaled`; nothing is done where *skip is set (a Krylov breakdown).
-// A warp per configuration; the matrix elements and targets are read once, past L1
-// (14400 determinants: 312 MB, 48 us at the measured HBM rate).  Four strides of loads
-// in flight per lane, where one load waited for the one before: 71.7 -> 59.7 us there,
-// 11.8 -> 10.2 us for 3136 determinants (cold caches).
-__global__ void __launch_bounds__(128) sigma_kernel(const long long* __restrict__ doff,
-                                                    const int* __restrict__ dhop,
-                                                    const double2* __restrict__ xpot,
-                                                    const long long* __restrict__ soff,
-                                                    const int* __restrict__ shop,
-                                                    const double2* __restrict__ xone,
-                                                    const double2* __restrict__ xz, double ez,
-                                                    double diag, const double2* __restrict__ in,
-                                                    int nc, double2* __restrict__ out, double2 tf, int scaled,
-                                                    const int* __restrict__ skip) {
+// sigma(c1) = const A(c1) + sum_dhops xpot A(dhop) + sum_shops (xone + ez xz) A(shop) + ez nucdip A(c1).
+// With `skip` given, times `tf`, and nothing is done where *skip is set (a Krylov breakdown).
+// Filled up to 160 bytes: the host's share of a launch depends on the size of the argument
+// block (96 or 160 bytes 2.1 us, 104 to 128, 256 or 512 bytes 2.85), and it is the bound of
+// the products of a tiny space, which take the device 2.2 us.
+struct SigmaArgs {
+  const long long* doff;
+  const int* dhop;
+  const double2* xpot;
+  const long long* soff;
+  const int* shop;
+  const double2* xone;
+  const double2* xz;
+  double ez, diag;
+  const double2* in;
+  double2* out;
+  double2 tf;
+  const int* skip;
+  int nc;
+  char fill[36];
+};
+static_assert(sizeof(SigmaArgs) == 160, "the size that the host launches faster");
+// A warp per configuration, four strides of loads in flight per lane (one load waited for
+// the one before: 14400 determinants 71.7 us, now 59.7, cold caches; 48 us is its 312 MB at
+// the measured HBM rate).  STREAM: see kSigmaKeep.
+template <bool STREAM>
+__global__ void __launch_bounds__(128) sigma_kernel(const __grid_constant__ SigmaArgs s) {
+  const double2* __restrict__ in = s.in;
   const int c1 = blockIdx.x * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (c1 >= nc || (skip && *skip)) return;
+  if (c1 >= s.nc || (s.skip && *s.skip)) return;
   double2 acc = make_double2(0.0, 0.0);
-  if (xpot)
-    acc = hop_sum<4>(doff[c1] + lane, doff[c1 + 1], dhop, [&](long long h) { return __ldcs(xpot + h); }, in);
-  double2 acc1 = hop_sum<2>(soff[c1] + lane, soff[c1 + 1], shop,
-                            [&](long long h) {
-                              double2 m = xone ? __ldcs(xone + h) : make_double2(0.0, 0.0);
-                              if (ez != 0.0) {
-                                const double2 z = __ldcs(xz + h);
-                                m.x = fma(ez, z.x, m.x);
-                                m.y = fma(ez, z.y, m.y);
-                              }
-                              return m;
-                            },
-                            in);
+  if (s.xpot)
+    acc = hop_sum<4, STREAM>(s.doff[c1] + lane, s.doff[c1 + 1], s.dhop,
+                             [&](long long h) { return load_hop<STREAM>(s.xpot + h); }, in);
+  double2 acc1 = hop_sum<2, STREAM>(s.soff[c1] + lane, s.soff[c1 + 1], s.shop,
+                                    [&](long long h) {
+                                      double2 m = s.xone ? load_hop<STREAM>(s.xone + h) : make_double2(0.0, 0.0);
+                                      if (s.ez != 0.0) {
+                                        const double2 z = load_hop<STREAM>(s.xz + h);
+                                        m.x = fma(s.ez, z.x, m.x);
+                                        m.y = fma(s.ez, z.y, m.y);
+                                      }
+                                      return m;
+                                    },
+                                    in);
   acc = warp_sum(acc);
   acc1 = warp_sum(acc1);
   if (lane == 0) {
     const double2 a = in[c1];
-    double2 r = make_double2(diag * a.x, diag * a.y);
+    double2 r = make_double2(s.diag * a.x, s.diag * a.y);
     r = cadd(r, acc);
     r = cadd(r, acc1);
-    out[c1] = scaled ? cmul(tf, r) : r;
+    s.out[c1] = s.skip ? cmul(s.tf, r) : r;
   }
 }
 
@@ -613,7 +631,7 @@ struct HopSum {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const bool ok = h + D * u < e;
-      t[u] = ok ? __ldcs(hop + h + D * u) : -1;
+      t[u] = ok ? __ldg(hop + h + D * u) : -1;
       m[u] = ok ? mat(h + D * u) : make_double2(0.0, 0.0);
     }
   }
@@ -641,77 +659,77 @@ struct HopSum {
 // kernel took some 10 with its launch.
 constexpr int kSigmaWarps = 148 * 24;
 template <int W>
-__global__ void __launch_bounds__(128, 6) sigma_small_kernel(const long long* __restrict__ doff,
-                                                             const int* __restrict__ dhop,
-                                                             const double2* __restrict__ xpot,
-                                                             const long long* __restrict__ soff,
-                                                             const int* __restrict__ shop,
-                                                             const double2* __restrict__ xone,
-                                                             const double2* __restrict__ xz, double ez, double diag,
-                                                             const double2* in, int nc, double2* out, double2 tf,
-                                                             int scaled, const int* skip) {
+__global__ void __launch_bounds__(128, 6) sigma_small_kernel(const __grid_constant__ SigmaArgs s) {
   __shared__ double2 part[4];
   const int warp = threadIdx.x >> 5, l = threadIdx.x % (32 * W);
   const int c1 = blockIdx.x * (4 / W) + warp / W;
-  const bool ok = c1 < nc;
-  auto two = [&](long long h) { return __ldcs(xpot + h); };
+  const bool ok = c1 < s.nc;
+  auto two = [&](long long h) { return __ldg(s.xpot + h); };
   auto one = [&](long long h) {
-    double2 m = xone ? __ldcs(xone + h) : make_double2(0.0, 0.0);
-    if (ez != 0.0) {
-      const double2 z = __ldcs(xz + h);
-      m.x = fma(ez, z.x, m.x);
-      m.y = fma(ez, z.y, m.y);
+    double2 m = s.xone ? __ldg(s.xone + h) : make_double2(0.0, 0.0);
+    if (s.ez != 0.0) {
+      const double2 z = __ldg(s.xz + h);
+      m.x = fma(s.ez, z.x, m.x);
+      m.y = fma(s.ez, z.y, m.y);
     }
     return m;
   };
   HopSum<8 / W, 32 * W> d;
-  HopSum<1, 32 * W> s;
-  d.h = d.e = s.h = s.e = 0;
+  HopSum<1, 32 * W> o;
+  d.h = d.e = o.h = o.e = 0;
   if (ok) {
-    if (xpot) {
-      d.h = doff[c1] + l;
-      d.e = doff[c1 + 1];
+    if (s.xpot) {
+      d.h = s.doff[c1] + l;
+      d.e = s.doff[c1 + 1];
     }
-    s.h = soff[c1] + l;
-    s.e = soff[c1 + 1];
+    o.h = s.soff[c1] + l;
+    o.e = s.soff[c1 + 1];
   }
-  d.load(dhop, two);
-  s.load(shop, one);
+  d.load(s.dhop, two);
+  o.load(s.shop, one);
   grid_dependents_launch();
   grid_dependency_wait();
-  if (skip && *skip) return;
-  double2 acc = warp_sum(cadd(d.sum(dhop, two, in), s.sum(shop, one, in)));
+  if (s.skip && *s.skip) return;
+  double2 acc = warp_sum(cadd(d.sum(s.dhop, two, s.in), o.sum(s.shop, one, s.in)));
   if (W > 1) {
     if ((threadIdx.x & 31) == 0) part[warp] = acc;
     __syncthreads();
   }
   if (l == 0 && ok) {
-    const double2 a = in[c1];
-    double2 r = make_double2(diag * a.x, diag * a.y);
+    const double2 a = s.in[c1];
+    double2 r = make_double2(s.diag * a.x, s.diag * a.y);
     if (W > 1) {
 #pragma unroll
       for (int w = 0; w < W; ++w) r = cadd(r, part[warp + w]);
     } else {
       r = cadd(r, acc);
     }
-    out[c1] = scaled ? cmul(tf, r) : r;
+    s.out[c1] = s.skip ? cmul(s.tf, r) : r;
   }
 }
 
+// Hops (16 + 4 bytes) of more than kSigmaKeep are read past the caches (evict first): the
+// vector keeps its place there, and nothing is lost, since they would not stay in the
+// 126 MB L2 until the next product.  Fewer are kept in it, as a driver's own propagator and
+// the Krylov chain come back to them at once.  us per product, one after another / with L2
+// flushed before each, evict first against kept: 72 MB (6084 determinants) 20.8 / 37.0
+// against 19.0 / 40.1 and, waiting for each, 33.7 against 28.6; 117 MB (8281) 28.6 / 42.5
+// against 30.8 / 49.5; 43 MB (4356) 12.3 / 26.2 against 10.4 / 27.4.
+constexpr long long kSigmaBytes = 20, kSigmaKeep = 96LL << 20;
 // `early`: a small space's kernel may start before the one in front has ended
 static int launch_sigma(Ctx& c, bool early, const double2* xpot, const double2* xone, double ez, double diag,
-                        const double2* in, double2* out, double2 tf, bool scaled, const int* skip) {
-  CIState& s = c.ci;
+                        const double2* in, double2* out, double2 tf, const int* skip) {
+  const CIState& s = c.ci;
+  const SigmaArgs a{s.dhop_off, s.dhop, xpot, s.shop_off, s.shop, xone, s.xz, ez, diag, in, out, tf, skip, s.nc};
   if (s.nc > kSigmaWarps) {
-    sigma_kernel<<<ceil_div(s.nc, 4), 128, 0, c.stream>>>(s.dhop_off, s.dhop, xpot, s.shop_off, s.shop, xone, s.xz, ez,
-                                                          diag, in, s.nc, out, tf, scaled ? 1 : 0, skip);
+    const auto kernel = kSigmaBytes * (s.ndh + s.nsh) > kSigmaKeep ? sigma_kernel<true> : sigma_kernel<false>;
+    kernel<<<ceil_div(s.nc, 4), 128, 0, c.stream>>>(a);
     SG_LAUNCHED();
     return SINCGPU_OK;
   }
   const bool four = s.nc <= kSigmaWarps / 4;
   return launch_waiting(c.stream, early, four ? sigma_small_kernel<4> : sigma_small_kernel<1>,
-                        dim3(ceil_div(s.nc, four ? 1 : 4)), dim3(128), 0, s.dhop_off, s.dhop, xpot, s.shop_off, s.shop,
-                        xone, s.xz, ez, diag, in, s.nc, out, tf, scaled ? 1 : 0, skip);
+                        dim3(ceil_div(s.nc, four ? 1 : 4)), dim3(128), 0, a);
 }
 
 // z-dipole expectation (dipolesub_one, MCTDH.SRC/dipolesub.f90:20-125, z part):
@@ -719,7 +737,7 @@ static int launch_sigma(Ctx& c, bool early, const double2* xpot, const double2* 
 int ci_dipole_z(Ctx& c, const double2* a, double2* tmp, double nucdipz, double2* dip, double* normsq) {
   CIState& s = c.ci;
   SG_CHECK(s.attached && s.assembled, SINCGPU_ESTATE, "sparse CI matrices not assembled");
-  SG_TRY(launch_sigma(c, false, nullptr, nullptr, 1.0, 0.0, a, tmp, make_double2(1.0, 0.0), false, nullptr));
+  SG_TRY(launch_sigma(c, false, nullptr, nullptr, 1.0, 0.0, a, tmp, make_double2(1.0, 0.0), nullptr));
   std::vector<double2> ha(s.nc), za(s.nc);
   SG_CUDA(cudaMemcpyAsync(ha.data(), a, sizeof(double2) * s.nc, cudaMemcpyDeviceToHost, c.stream));
   SG_CUDA(cudaMemcpyAsync(za.data(), tmp, sizeof(double2) * s.nc, cudaMemcpyDeviceToHost, c.stream));
@@ -747,8 +765,7 @@ int ci_sigma(Ctx& c, const double2* in, double2* out, double constant, double ez
   SG_CHECK(s.attached && s.assembled, SINCGPU_ESTATE, "sparse CI matrices not assembled");
   ProfScope ps(c, ST_CI);
   // in a Krylov chain the kernel in front writes `in` and the flag
-  return launch_sigma(c, skip != nullptr, s.xpot, s.xone, ez, constant + ez * nucdipz, in, out, tf, skip != nullptr,
-                      skip);
+  return launch_sigma(c, skip != nullptr, s.xpot, s.xone, ez, constant + ez * nucdipz, in, out, tf, skip);
 }
 
 }  // namespace sincgpu
