@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(DMMA ? 64 * R : 256, 1) twoe_gemm3_kernel(cons
 // blocks on and below the diagonal are computed, R (2R + 1) of the (2R)^2; each
 // off-diagonal block is also stored transposed in place of its mirror.  Row blocks p and 2R - 1 - p form a pair
 // with 2R + 1 blocks; warp 2p takes the first R + 1 of them, warp 2p + 1 the rest.
-template <int R, bool SYM, int KT>
+template <int R, bool SYM, int KT, bool ROWS>
 __global__ void __launch_bounds__(64 * R, 1) twoe_dmma_kernel(const double2* __restrict__ phi1,
                                                               const double2* __restrict__ phi2,
                                                               const int* __restrict__ pa, const int* __restrict__ pb,
@@ -247,7 +247,10 @@ __global__ void __launch_bounds__(64 * R, 1) twoe_dmma_kernel(const double2* __r
   int* sa = reinterpret_cast<int*>(fsm + 6 * nspf * KT);
   int* sb = sa + TT;
   int* sc = sb + TT;
-  __shared__ int srow[TT];  // the tile's columns' rows of Rpl, -1 beyond M
+  // the tile's columns' rows of Rpl, -1 beyond M (ROWS: the rows in use are listed; else
+  // they are all rows in order, and the table's read would delay every copy's address: the
+  // contraction of 81 pairs at 33^3 100.8 us without it, 106.7 with)
+  __shared__ int srow[ROWS ? TT : 1];
   // tile (tm, tn): SYM CTAs take the diagonal tiles (blockIdx.x = tm = tn); the
   // others the upper-triangle tiles, the diagonal included unless `strict`
   int tm = 0, tn = 0;
@@ -267,9 +270,9 @@ __global__ void __launch_bounds__(64 * R, 1) twoe_dmma_kernel(const double2* __r
   const int tid = threadIdx.x;
   for (int i = tid; i < TT; i += NTH) {
     const int m = m0 + i;
-    srow[i] = n0 + i < M ? (rows ? rows[n0 + i] : n0 + i) : -1;
+    if (ROWS) srow[i] = n0 + i < M ? rows[n0 + i] : -1;
     if (m < M) {
-      const int r = rows ? rows[m] : m, p = r % npair;
+      const int r = ROWS ? rows[m] : m, p = r % npair;
       sa[i] = pa[p];
       sb[i] = pb[p];
       sc[i] = r / npair;
@@ -295,7 +298,7 @@ __global__ void __launch_bounds__(64 * R, 1) twoe_dmma_kernel(const double2* __r
     double* b = Bs + st * TT * TS;
     for (int i = tid; i < KT * TT; i += NTH) {
       const int nn = i / KT, k = i % KT;
-      const int r = srow[nn];
+      const int r = ROWS ? srow[nn] : n0 + nn < M ? n0 + nn : -1;
       const long long x = x0 + k;
       const bool ok = r >= 0 && x < xe;
       cp_async8(&b[nn * TS + k], ok ? (const void*)(Rpl + (long long)r * G + x) : (const void*)Rpl, ok);
@@ -617,17 +620,26 @@ static size_t twoe_pipe_smem(int R, int KT, int n) {
 }
 constexpr int kTwoeSmemMax = 226 * 1024;  // (the kernels' static tables beside it)
 
-template <int RR, bool SYM, int KT>
+template <int RR, bool SYM, int KT, bool ROWS>
 static int launch_twoe_pipe_t(Ctx& c, dim3 grid, size_t bytes, const double2* phi1, const double2* phi2,
                               const int* d_pa, const int* d_pb, const double* Rpl, const int* d_rows, int M,
                               int npair, int ntn, long long xper, double* part, int strict) {
   // process-wide attribute, one fixed value (thread-safe static initialisation)
-  static const cudaError_t attr = cudaFuncSetAttribute(twoe_dmma_kernel<RR, SYM, KT>,
+  static const cudaError_t attr = cudaFuncSetAttribute(twoe_dmma_kernel<RR, SYM, KT, ROWS>,
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, kTwoeSmemMax);
   SG_CUDA(attr);
-  twoe_dmma_kernel<RR, SYM, KT><<<grid, 64 * RR, bytes, c.stream>>>(phi1, phi2, d_pa, d_pb, Rpl, d_rows, M, npair,
-                                                                     c.nspf, c.G, ntn, xper, part, strict);
+  twoe_dmma_kernel<RR, SYM, KT, ROWS><<<grid, 64 * RR, bytes, c.stream>>>(
+      phi1, phi2, d_pa, d_pb, Rpl, d_rows, M, npair, c.nspf, c.G, ntn, xper, part, strict);
   return SINCGPU_OK;
+}
+template <int RR, int KT>
+static int launch_twoe_pipe_k(Ctx& c, dim3 grid, bool sym, const double2* phi1, const double2* phi2, const int* d_pa,
+                              const int* d_pb, const double* Rpl, const int* d_rows, int M, int npair, int ntn,
+                              long long xper, double* part, int strict) {
+  const auto launch = d_rows ? (sym ? launch_twoe_pipe_t<RR, true, KT, true> : launch_twoe_pipe_t<RR, false, KT, true>)
+                             : (sym ? launch_twoe_pipe_t<RR, true, KT, false> : launch_twoe_pipe_t<RR, false, KT, false>);
+  return launch(c, grid, twoe_pipe_smem(RR, KT, c.nspf), phi1, phi2, d_pa, d_pb, Rpl, d_rows, M, npair, ntn, xper, part,
+                sym ? 0 : strict);
 }
 
 // K stages of 32 points where the shared memory allows (half the stages and
@@ -636,16 +648,9 @@ template <int RR>
 static int launch_twoe_pipe(Ctx& c, dim3 grid, bool sym, const double2* phi1, const double2* phi2,
                             const int* d_pa, const int* d_pb, const double* Rpl, const int* d_rows, int M,
                             int npair, int ntn, long long xper, double* part, int strict = 0) {
-  const size_t b32 = twoe_pipe_smem(RR, 32, c.nspf), b16 = twoe_pipe_smem(RR, 16, c.nspf);
-  if (b32 <= (size_t)kTwoeSmemMax)
-    return sym ? launch_twoe_pipe_t<RR, true, 32>(c, grid, b32, phi1, phi2, d_pa, d_pb, Rpl, d_rows, M, npair, ntn, xper, part,
-                                                  0)
-               : launch_twoe_pipe_t<RR, false, 32>(c, grid, b32, phi1, phi2, d_pa, d_pb, Rpl, d_rows, M, npair, ntn, xper,
-                                                   part, strict);
-  return sym ? launch_twoe_pipe_t<RR, true, 16>(c, grid, b16, phi1, phi2, d_pa, d_pb, Rpl, d_rows, M, npair, ntn, xper, part,
-                                                0)
-             : launch_twoe_pipe_t<RR, false, 16>(c, grid, b16, phi1, phi2, d_pa, d_pb, Rpl, d_rows, M, npair, ntn, xper, part,
-                                                 strict);
+  const auto launch = twoe_pipe_smem(RR, 32, c.nspf) <= (size_t)kTwoeSmemMax ? launch_twoe_pipe_k<RR, 32>
+                                                                             : launch_twoe_pipe_k<RR, 16>;
+  return launch(c, grid, sym, phi1, phi2, d_pa, d_pb, Rpl, d_rows, M, npair, ntn, xper, part, strict);
 }
 
 static void pair_lut(int n, const int* pa, const int* pb, int npair, bool herm, std::vector<int>& lut) {
