@@ -17,6 +17,7 @@
 #include <cooperative_groups.h>
 #include "context.hpp"
 #include "dmma.cuh"
+#include "gram_schmidt.cuh"
 
 namespace sincgpu {
 
@@ -94,12 +95,9 @@ __global__ void __launch_bounds__(kKryThreads) kry_mgs_kernel(double* __restrict
 }
 
 // One Arnoldi step's orthogonalisation on a thread-block cluster: the modified
-// Gram-Schmidt coefficients from one pass of dots.  With r_i = <v_i, p> and
-// L_ik = <v_i, v_k> (k < i; rounding level), the sequential projections' h solve
-// (I + L) h = r, so h = r - L r up to L^2, which is far below rounding (L is some
-// eps / break_tol at most): the same coefficients and the same loss of orthogonality
-// as kry_mgs_kernel to rounding, without its j + 1 dependent sums.  Row j of L is
-// formed in the same pass over V (v_j is a row already) and kept for later steps.
+// Gram-Schmidt coefficients from one pass of dots (gs_coefficients) instead of
+// kry_mgs_kernel's j + 1 dependent sums.  Row j of L is formed in the same pass over V (v_j
+// is a row already).
 //
 // CTA q of the cluster owns the slice [q S, q S + S) of the vectors, S = ceil(n /
 // kGsCluster) rounded up to even; p, v_j and the first `cap` rows of the slice sit in
@@ -110,15 +108,16 @@ __global__ void __launch_bounds__(kKryThreads) kry_mgs_kernel(double* __restrict
 // two cluster barriers.  The rows' way into shared memory comes before the wait for the
 // sigma product that writes p: that product and the step before may still run (512
 // threads, so that all fit an SM).  After the wait, at 25 rows of 3136 determinants: loads
-// 0.8 us, dots 2.2, barrier 0.7, coefficients 1.1, update 0.9, norm 1.2.  One A-vector step
-// of 30 vectors at 3136 determinants, launches included: 810 -> 515 us, of which clusters of
-// 8 whose rows came from L2 after the sigma product had ended took 14 us a vector; CMF step
-// at 31^3 14.3 -> 12.1 ms.
+// 0.8 us, dots 2.2, barrier 0.7, coefficients 1.5, update 0.9, norm 1.2.  One A-vector step
+// of 30 vectors at 3136 determinants, launches included: 810 -> 527 us, of which clusters of
+// 8 whose rows came from L2 after the sigma product had ended took 14 us a vector.  One CTA
+// with sequential projections is slower at every size: 25 determinants 0.87 ms a step of up
+// to 30 vectors, 0.35 on the cluster; 450 0.95 and 0.38; 3136 1.57 and 0.53.
 constexpr int kGsCluster = 16;
 constexpr int kGsThreads = 32 * kGsCluster;
 constexpr long long kGsSlice = 8100;    // most values of a slice
-constexpr long long kGsValues = 23900;  // of dynamic shared memory: p, v_j, rows of L, rows of V
-static_assert(2 * kGsSlice + kMaxKry * (kMaxKry - 1) / 2 <= kGsValues, "p, v_j and L must fit");
+constexpr long long kGsValues = 23900;  // of dynamic shared memory: p, v_j, rows of T, rows of V
+static_assert(2 * kGsSlice + kMaxKry * (kMaxKry - 1) / 2 <= kGsValues, "p, v_j and T must fit");
 
 __device__ __forceinline__ void cp_async16(double* smem, const double* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem));
@@ -171,11 +170,11 @@ __device__ __forceinline__ void gs_dots(int i0, int last, int half, int len, con
 // ALL: cap = j, every row in shared memory
 template <bool ALL>
 __global__ void __launch_bounds__(kGsThreads) kry_gs_kernel(double* V, long long n, int S, int cap, int j,
-                                                            double* Hm, int mh, double* Lm, double break_tol,
+                                                            double* Hm, int mh, double* Tm, double break_tol,
                                                             KryState* st) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
-  extern __shared__ __align__(16) double gsm[];  // p, v_j, rows 0 .. cap - 1 of the slice, rows of L
+  extern __shared__ __align__(16) double gsm[];  // p, v_j, rows 0 .. cap - 1 of the slice, rows of T
   __shared__ double2 part[kGsCluster][128];  // every CTA's partial dots <v_i, p>, <v_i, v_j>
   __shared__ double2 dots[2][128];           // this CTA's, by halves of its slice
   __shared__ double npart[kGsCluster], red[kGsThreads / 32], r[128], lrow[128], h[128];
@@ -184,20 +183,20 @@ __global__ void __launch_bounds__(kGsThreads) kry_gs_kernel(double* V, long long
   const long long lo = (long long)rank * S;
   const int len = (int)max(0LL, min((long long)S, n - lo));
   double* ps = gsm;
-  double* Ls = gsm + (long long)(2 + cap) * S;  // row i from i (i - 1) / 2
+  double* Ts = gsm + (long long)(2 + cap) * S;  // row i from i (i - 1) / 2
   double* pg = V + (long long)(j + 1) * n + lo;
   auto row = [&](int i) -> const double* {
     if (ALL) return gsm + (i == j ? 1 : 2 + i) * S;
     return i == j ? gsm + S : i < cap ? gsm + (long long)(2 + i) * S : V + (long long)i * n + lo;
   };
-  // Before the wait: rows 0 .. j - 1 of V and 0 .. j - 2 of L, all of steps that have ended
+  // Before the wait: rows 0 .. j - 1 of V and 0 .. j - 2 of T, all of steps that have ended
   // (the step in front waits for its own predecessor before it lets this one start).
   // Rows as pairs: n, S and so every len are even.
   for (int i = warp; i < cap; i += kGsThreads / 32)
     for (int k = 2 * lane; k < len; k += 64)
       cp_async16(gsm + (long long)(2 + i) * S + k, V + (long long)i * n + lo + k);
   for (int i = warp; i < j - 1; i += kGsThreads / 32)
-    for (int k = lane; k < i; k += 32) Ls[i * (i - 1) / 2 + k] = __ldcg(Lm + (long long)i * mh + k);
+    for (int k = lane; k < i; k += 32) Ts[i * (i - 1) / 2 + k] = __ldcg(Tm + (long long)i * mh + k);
   cp_async_wait_all();
   cl.sync();  // the CTAs whose shared memory is written are there
   grid_dependency_wait();
@@ -208,7 +207,7 @@ __global__ void __launch_bounds__(kGsThreads) kry_gs_kernel(double* V, long long
     ps[k] = __ldcg(pg + k);
     gsm[S + k] = __ldcg(vj + k);
   }
-  if (tid < j - 1) Ls[(j - 1) * (j - 2) / 2 + tid] = __ldcg(Lm + (long long)(j - 1) * mh + tid);
+  if (tid < j - 1) Ts[(j - 1) * (j - 2) / 2 + tid] = __ldcg(Tm + (long long)(j - 1) * mh + tid);
   __syncthreads();
   if (brk_before) return;
   for (int base = 0; base <= j; base += 32) {
@@ -228,25 +227,18 @@ __global__ void __launch_bounds__(kGsThreads) kry_gs_kernel(double* V, long long
     const double2 sum = cadd(a[0], a[1]);
     r[tid] = sum.x;
     lrow[tid] = sum.y;  // row j of L (its diagonal is not used)
-    if (rank == 0 && tid < j) Lm[(long long)j * mh + tid] = sum.y;
   }
   __syncthreads();
-  // h_i = r_i - sum_{k < i} L_ik r_k, a warp per row, the same in every CTA
-  for (int i = warp; i <= j; i += kGsThreads / 32) {
-    const double* L = i < j ? Ls + i * (i - 1) / 2 : lrow;
-    double a = 0.0;
-    for (int k = lane; k < i; k += 32) a = fma(L[k], r[k], a);
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-    if (lane == 0) {
-      h[i] = r[i] - a;
-      if (rank == 0) Hm[(long long)j * mh + i] = r[i] - a;
-    }
-  }
-  __syncthreads();
+  // the same in every CTA
+  const double hj = gs_coefficients(
+      j, h, [&](int i) { return r[i]; }, [&](int k) { return lrow[k]; },
+      [&](int i, int k) { return Ts[i * (i - 1) / 2 + k]; }, rank, kGsCluster,
+      [&](int k, double v) { Tm[(long long)j * mh + k] = v; });
+  if (rank == 0 && tid <= j) Hm[(long long)j * mh + tid] = tid < j ? h[tid] : hj;
   double s = 0.0;
   const int staged = ALL ? j : cap;
   for (int k = tid; k < len; k += kGsThreads) {
-    double x[4] = {fma(-h[j], gsm[S + k], ps[k]), 0.0, 0.0, 0.0};
+    double x[4] = {fma(-hj, gsm[S + k], ps[k]), 0.0, 0.0, 0.0};
     int i = 0;
 #pragma unroll 2
     for (; i + 4 <= staged; i += 4)
@@ -557,8 +549,8 @@ int expv_avector(Ctx& c, const double2* v, double2* w, double t, double2 timefac
   double* Hm = V + (size_t)(m + 2) * n;
   double* exph = Hm + (size_t)mh * mh;
   double* pscr = exph + 128;
-  double* Lm = pscr + 5 * (size_t)mh * mh;  // dots of the Krylov vectors (kry_gs_kernel)
-  KryState* dst = (KryState*)(Lm + (size_t)mh * mh);
+  double* Tm = pscr + 5 * (size_t)mh * mh;  // kry_gs_kernel's T
+  KryState* dst = (KryState*)(Tm + (size_t)mh * mh);
   int* d_ns = (int*)(dst + 1);
   int nmult = 0;
   const double delta = 1.2, gamma = 0.9, break_tol = 1.0e-7;
@@ -604,7 +596,7 @@ int expv_avector(Ctx& c, const double2* v, double2* w, double t, double2 timefac
         const long long tri = j * (j - 1) / 2;
         const int cap = (int)std::min<long long>(j, (kGsValues - tri) / S - 2);
         SG_TRY(launch_gs_cluster(c, cap == j ? kry_gs_kernel<true> : kry_gs_kernel<false>, kGsThreads, sizeof(double) * ((2 + cap) * (size_t)S + tri), true, V,
-                                 n, (int)S, cap, j, Hm, mh, Lm, break_tol, dst));
+                                 n, (int)S, cap, j, Hm, mh, Tm, break_tol, dst));
       } else {
         kry_mgs_kernel<<<1, kKryThreads, 0, c.stream>>>(V, n, j, Hm, mh, break_tol, dst);
         SG_LAUNCHED();

@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <cmath>
 #include "context.hpp"
+#include "gram_schmidt.cuh"
 #include "jacobi_svd.cuh"
 
 namespace sincgpu {
@@ -266,9 +267,8 @@ __global__ void __launch_bounds__(kLvThreads, 2) lv_arnoldi_orth_kernel(const do
 
 // The orthogonalisation of Arnoldi step j in three launches of any length (option
 // orth_onepass): the coefficients of the modified Gram-Schmidt from one pass of dots.
-// With r_i = <v_i, p> and L_ik = <v_i, v_k> (k < i; rounding level), the sequential
-// projections' h solve (I + L) h = r, so h = r - L r up to L^2, which is far below
-// rounding.  Row j of L is summed in the same pass (v_j is a row already) and kept.
+// With r_i = <v_i, p> and row j of L, <v_j, v_k>, summed in one pass (v_j is a row already),
+// gs_coefficients forms them.
 //   lv_dots_all: r and row j of L, eight rows of V at a time in registers; the last CTA
 //                adds the partials in a fixed order and forms h
 //   lv_project:  p -= sum_i h_i v_i and |p|^2; the last CTA sets h(j+1,j) and breakdown
@@ -294,10 +294,10 @@ __device__ __forceinline__ bool lv_last_cta(unsigned* count, unsigned* sh) {
   return *sh != 0;
 }
 
-// totals of the 2 (j + 1) dots over the CTAs' partials in a fixed order, row j of L (to
-// Lm when `keep`) and the coefficients h; one CTA
-__device__ __forceinline__ void lv_coefficients(const double* part, int j, double* tot, double* h, double* Lm, int mh,
-                                                bool keep) {
+// totals of the 2 (j + 1) dots over the CTAs' partials in a fixed order, the coefficients h
+// and elements k0, k0 + kstep, ... of row j of T; one CTA
+__device__ __forceinline__ void lv_coefficients(const double* part, int j, double* tot, double* h, double* Tm, int mh,
+                                                int k0, int kstep) {
   constexpr int U = (kLvBlocks + 31) / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int e = warp; e < 2 * (j + 1); e += kLvThreads / 32) {
@@ -308,25 +308,21 @@ __device__ __forceinline__ void lv_coefficients(const double* part, int j, doubl
 #pragma unroll
     for (int u = 0; u < U; ++u) s += v[u];
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) {
-      tot[e] = s;
-      if (keep && (e & 1) && e / 2 < j) Lm[(long long)j * mh + e / 2] = s;
-    }
+    if (lane == 0) tot[e] = s;
   }
   __syncthreads();
-  for (int i = warp; i <= j; i += kLvThreads / 32) {
-    double a = 0.0;
-    for (int k = lane; k < i; k += 32) a = fma(i < j ? Lm[(long long)i * mh + k] : tot[2 * k + 1], tot[2 * k], a);
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-    if (lane == 0) h[i] = tot[2 * i] - a;
-  }
+  const double hj = gs_coefficients(
+      j, h, [&](int i) { return tot[2 * i]; }, [&](int k) { return tot[2 * k + 1]; },
+      [&](int i, int k) { return Tm[(long long)i * mh + k]; }, k0, kstep,
+      [&](int k, double v) { Tm[(long long)j * mh + k] = v; });
+  if (threadIdx.x == 0) h[j] = hj;
   __syncthreads();
 }
 
 __global__ void __launch_bounds__(kLvThreads, 2) lv_dots_all_kernel(const double2* __restrict__ V,
                                                                      const double2* __restrict__ p, long long nv, int j,
                                                                      double* __restrict__ part, double* __restrict__ Hm,
-                                                                     int mh, double* __restrict__ Lm,
+                                                                     int mh, double* __restrict__ Tm,
                                                                      const OrbKryState* __restrict__ st,
                                                                      unsigned* __restrict__ count) {
   __shared__ double red[kLvThreads / 32][2 * kRows];
@@ -372,7 +368,7 @@ __global__ void __launch_bounds__(kLvThreads, 2) lv_dots_all_kernel(const double
     }
   }
   if (!lv_last_cta(count, &last)) return;
-  lv_coefficients(part, j, tot, h, Lm, mh, true);
+  lv_coefficients(part, j, tot, h, Tm, mh, 0, 1);
   if (tid <= j) Hm[(long long)j * mh + tid] = h[tid];
 }
 
@@ -384,7 +380,7 @@ __global__ void __launch_bounds__(kLvThreads, 2) lv_dots_all_kernel(const double
 template <int E>
 __global__ void __launch_bounds__(kLvThreads, 2) lv_orth_onepass_kernel(const double2* __restrict__ V, double2* p,
                                                                          long long nv, int j, double* part, double* partn,
-                                                                         double* __restrict__ Hm, int mh, double* Lm,
+                                                                         double* __restrict__ Hm, int mh, double* Tm,
                                                                          double break_tol, OrbKryState* st,
                                                                          unsigned* bar, OrbKryState* host) {
   constexpr int R = 4;  // rows of V in registers at a time
@@ -440,7 +436,7 @@ __global__ void __launch_bounds__(kLvThreads, 2) lv_orth_onepass_kernel(const do
     if (tid == 0) host->gfail = 1;
     return;
   }
-  lv_coefficients(part, j, tot, h, Lm, mh, blockIdx.x == 0);
+  lv_coefficients(part, j, tot, h, Tm, mh, blockIdx.x, gridDim.x);
   if (blockIdx.x == 0 && tid <= j) Hm[(long long)j * mh + tid] = h[tid];
   double s = 0.0;
   for (int c0 = j / R * R; c0 >= 0; c0 -= R)  // the rows read last are still in L2
@@ -664,7 +660,7 @@ struct OrbWork {
   double2 *V, *jv, *jvo, *u, *w, *T, *tmp, *dpart;
   double2 *D2, *M1, *ovl, *smh;
   double *part0, *part1, *Hm, *exph, *Efull, *pscratch, *err;
-  double *gpart, *Lm;  // lv_dots_all_kernel's partials and the dots of the Krylov vectors
+  double *gpart, *Tm;  // lv_dots_all_kernel's partials, gs_coefficients' T
   OrbKryState* st;
   int* ns;
   unsigned* gbar;  // lv_arnoldi_orth_kernel's grid barrier (count, generation), lv_last_cta's count
@@ -707,7 +703,7 @@ int orb_work(Ctx& c, int m, OrbWork& o) {
   o.part0 = (double*)take(sizeof(double) * kLvBlocks);
   o.part1 = (double*)take(sizeof(double) * kLvBlocks);
   o.Hm = (double*)take(sizeof(double) * mh * mh);
-  o.Lm = (double*)take(sizeof(double) * mh * mh);
+  o.Tm = (double*)take(sizeof(double) * mh * mh);
   o.gpart = (double*)take(sizeof(double) * 2 * (m + 1) * kLvBlocks);
   o.exph = (double*)take(sizeof(double) * 130);
   o.Efull = (double*)take(sizeof(double) * kMaxPadeOrb * kMaxPadeOrb);
@@ -896,19 +892,19 @@ int expospfprop(Ctx& c, double2* phi, const MeanFieldSlot* slots, double tin, do
       if (c.orth_onepass && one_launch) {
         hst_pin->gfail = 0;  // no kernel that writes it is in flight
         const double2* Vc = o.V;
-        double *P0 = o.gpart, *P1 = o.part0, *H = o.Hm, *Lm = o.Lm;
+        double *P0 = o.gpart, *P1 = o.part0, *H = o.Hm, *Tm = o.Tm;
         OrbKryState* S = o.st;
         unsigned* B = o.gbar;
         int jj = j, mhh = mh;
         long long nvv = nv;
         double bt = break_tol;
         void* args[] = {(void*)&Vc,  (void*)&p,  (void*)&nvv, (void*)&jj, (void*)&P0, (void*)&P1,     (void*)&H,
-                        (void*)&mhh, (void*)&Lm, (void*)&bt,  (void*)&S,  (void*)&B,  (void*)&hst_pin};
+                        (void*)&mhh, (void*)&Tm, (void*)&bt,  (void*)&S,  (void*)&B,  (void*)&hst_pin};
         SG_CUDA(cudaLaunchCooperativeKernel((const void*)lv_orth_onepass_kernel<kOrthE>, dim3(lvg), dim3(kLvThreads),
                                             args, 0, c.stream));
         count_launch();
       } else if (c.orth_onepass) {
-        lv_dots_all_kernel<<<lvg, kLvThreads, 0, c.stream>>>(o.V, p, nv, j, o.gpart, o.Hm, mh, o.Lm, o.st, o.gbar + 2);
+        lv_dots_all_kernel<<<lvg, kLvThreads, 0, c.stream>>>(o.V, p, nv, j, o.gpart, o.Hm, mh, o.Tm, o.st, o.gbar + 2);
         SG_LAUNCHED();
         lv_project_kernel<<<lvg, kLvThreads, 0, c.stream>>>(o.V, p, nv, j, o.part0, o.Hm, mh, break_tol, o.st,
                                                             o.gbar + 2);
