@@ -311,27 +311,55 @@ __global__ void __launch_bounds__(kKryThreads) kry_update_cluster_kernel(const d
   cl.sync();  // no CTA leaves while its partial is read
 }
 
-// launch of a kernel on one cluster of kGsCluster CTAs; `early`: before the kernel in front
-// of it has ended
+// a launch on one cluster of kGsCluster CTAs; `early`: before the kernel in front of it has ended
+struct GsLaunch {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[2];
+  GsLaunch(int threads, size_t smem, cudaStream_t stream, bool early) {
+    cfg.gridDim = dim3(kGsCluster, 1, 1);
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kGsCluster;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = early ? 2 : 1;
+  }
+};
 template <class... KA, class... A>
 static int launch_gs_cluster(Ctx& c, void (*kernel)(KA...), int threads, size_t smem, bool early, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(kGsCluster, 1, 1);
-  cfg.blockDim = dim3(threads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = c.stream;
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = kGsCluster;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = early ? 2 : 1;
-  SG_CUDA(cudaLaunchKernelEx(&cfg, kernel, (KA)args...));
+  GsLaunch l(threads, smem, c.stream, early);
+  SG_CUDA(cudaLaunchKernelEx(&l.cfg, kernel, (KA)args...));
   count_launch();
   return SINCGPU_OK;
+}
+
+// Whether the device places the cluster kernels, with the most shared memory that they take:
+// 16 CTAs are more than every device has to place (8), and a part of one may hold fewer.
+// Sets the kernels' attributes; once per process.
+static bool gs_cluster_fits() {
+  static const bool fits = [] {
+    constexpr size_t smem = sizeof(double) * kGsValues;
+    for (auto k : {kry_gs_kernel<true>, kry_gs_kernel<false>}) {
+      int n = 0;
+      GsLaunch l(kGsThreads, smem, nullptr, false);
+      if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+          cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+          cudaOccupancyMaxActiveClusters(&n, k, &l.cfg) != cudaSuccess || n < 1)
+        return false;
+    }
+    int n = 0;
+    GsLaunch l(kKryThreads, 0, nullptr, false);
+    return cudaFuncSetAttribute(kry_update_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+               cudaSuccess &&
+           cudaOccupancyMaxActiveClusters(&n, kry_update_cluster_kernel, &l.cfg) == cudaSuccess && n >= 1;
+  }();
+  if (!fits) (void)cudaGetLastError();
+  return fits;
 }
 
 __global__ void __launch_bounds__(kKryThreads) kry_avnorm_kernel(const double* __restrict__ p, long long n,
@@ -569,18 +597,10 @@ int expv_avector(Ctx& c, const double2* v, double2* w, double t, double2 timefac
   KryState hst{};
   bool have_beta = false;
   ProfScope ps(c, ST_CI);
-  // the cluster kernels where a slice of p and v_j fits shared memory, else one CTA
+  // the cluster kernels where a slice of p and v_j fits shared memory and the device places
+  // them, else one CTA
   const long long S = ((n + kGsCluster - 1) / kGsCluster + 1) / 2 * 2;
-  const bool cluster = c.kry_cluster && S <= kGsSlice;
-  static const cudaError_t attr = [] {  // fixed values, set once
-    for (auto k : {kry_gs_kernel<true>, kry_gs_kernel<false>}) {
-      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(double) * kGsValues));
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-      if (e != cudaSuccess) return e;
-    }
-    return cudaFuncSetAttribute(kry_update_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  }();
-  SG_CUDA(attr);
+  const bool cluster = c.kry_cluster && S <= kGsSlice && gs_cluster_fits();
   while (t_now < t_out) {
     ++nstep;
     t_last = t_step;
