@@ -233,9 +233,10 @@ __global__ void __launch_bounds__(64 * R, 1) twoe_dmma_kernel(const double2* __r
                                                               const double2* __restrict__ phi2,
                                                               const int* __restrict__ pa, const int* __restrict__ pb,
                                                               const double* __restrict__ Rpl,
-                                                              const int* __restrict__ rows, int M, int npair,
+                                                              const int* __restrict__ rows, int nrow, int npair,
                                                               int nspf, long long G, int ntn, long long xper,
                                                               double* __restrict__ part, int strict) {
+  const int M = ROWS ? nrow : 2 * npair;  // (known even: the tile of 112 rows 70 us at 41^3, 74 without)
   constexpr int TT = 16 * R;
   constexpr int TS = KT + 4;  // shared-memory row stride (doubles), 4 mod 16
   constexpr int NTH = 64 * R;
@@ -298,9 +299,9 @@ __global__ void __launch_bounds__(64 * R, 1) twoe_dmma_kernel(const double2* __r
     double* b = Bs + st * TT * TS;
     for (int i = tid; i < KT * TT; i += NTH) {
       const int nn = i / KT, k = i % KT;
-      const int r = ROWS ? srow[nn] : n0 + nn < M ? n0 + nn : -1;
+      const int r = ROWS ? srow[nn] : n0 + nn;
       const long long x = x0 + k;
-      const bool ok = r >= 0 && x < xe;
+      const bool ok = (ROWS ? r >= 0 : r < M) && x < xe;
       cp_async8(&b[nn * TS + k], ok ? (const void*)(Rpl + (long long)r * G + x) : (const void*)Rpl, ok);
     }
     cp_async_commit();
@@ -688,21 +689,31 @@ int twoe_matel(Ctx& c, const double2* phi1, const double2* phi2, const int* h_pa
   SG_CHECK(n <= kMaxOrb, SINCGPU_ERANGE, "at most %d orbitals (got %d)", kMaxOrb, n);
   // the pipelined kernels copy whole complex values (16 bytes)
   const bool pipe = ((uintptr_t)phi1 % 16 == 0) && ((uintptr_t)phi2 % 16 == 0);
-  const bool drop = drop_rows(c, herm) && c.twoe_dmma && pipe;
+  // register block R (tile edge 16R): the one of 2..9 with the least padding of m rows (ties:
+  // the larger tile)
+  auto block = [&](int m) {
+    if (c.twoe_tile >= 2 && c.twoe_tile <= 9) return c.twoe_tile;
+    int R = 2;
+    for (int r = 2; r <= 9; ++r)
+      if (ceil_div(m, 16 * r) * 16 * r <= ceil_div(m, 16 * R) * 16 * R) R = r;
+    return R;
+  };
+  auto padded = [&](int m) { return ceil_div(m, 16 * block(m)) * 16 * block(m); };
+  // the diagonal pairs' zero rows are left out where that saves a tile's row of blocks (8, 11
+  // and 12 orbitals) or leads to the patches (13 to 16): in a tile of the same size the row
+  // table only delays the copies (57^3 / 3 orbitals 211 us with it, 198 without)
+  const int less = 2 * npair - n;
+  const bool patches = less > 144 && n <= kPatchOrb && c.twoe_tile == 0 && !c.twoe_symdiag;
+  const bool drop = drop_rows(c, herm) && c.twoe_dmma && pipe && (patches || padded(less) < padded(2 * npair));
   std::vector<int> rows, rowof;
   if (drop) hermitian_rows(h_pa, h_pb, npair, rows, rowof);
   const int M = drop ? (int)rows.size() : 2 * npair;
-  // register block R: the smallest of 2..9 whose 16R tile holds M, else 8 (multi-tile)
-  // tile edge 16R with the least padding of M (ties: the larger tile)
-  int R = 2;
-  for (int r = 2; r <= 9; ++r)
-    if (ceil_div(M, 16 * r) * 16 * r <= ceil_div(M, 16 * R) * 16 * R) R = r;
-  if (c.twoe_tile >= 2 && c.twoe_tile <= 9) R = c.twoe_tile;
+  const int R = block(M);
   // hermitian pairs in more rows than one tile (13 to 16 orbitals): patches of the triangle
   // (twoe_patch_kernel), up to the rows whose stages fit shared memory.  FP32 potentials
   // keep the tiles: their pair matrix is symmetric to 1e-8 only, so which half is formed
   // would show in the result.
-  const bool patch = drop && c.twoe_tile == 0 && !c.twoe_symdiag && M > 144 && n <= kPatchOrb;
+  const bool patch = drop && patches;
   const int npatch = ceil_div(M, kPatch) * (ceil_div(M, kPatch) + 1) / 2;
   const int groups = patch ? ceil_div(npatch, 16) : 1;  // CTAs that share the patches of a K range
   const int TT = patch ? kPatch : 16 * R;
