@@ -438,7 +438,9 @@ __global__ void __launch_bounds__(32 * kDotWarps) dots_mma_kernel(const double2*
   __threadfence();
   // thread (c, e) sums the c-th share of the CTAs for element e (consecutive threads,
   // consecutive elements; eight loads in flight), then the shares are added in order
-  const int nc = max(1, (int)blockDim.x / nn), per = ((int)gridDim.x + nc - 1) / nc;
+  // (eight a share at least: the shares of few elements are added one after another, 512 of
+  // one orbital's single element took 8 us)
+  const int nc = max(1, min((int)blockDim.x / nn, (int)gridDim.x / 8)), per = ((int)gridDim.x + nc - 1) / nc;
   double2* sh = reinterpret_cast<double2*>(dsm);  // [nc][nn]
   for (int q = tid; q < nc * nn; q += blockDim.x) {
     const int cc = q / nn, e = q - cc * nn, b1 = min((int)gridDim.x, (cc + 1) * per);
