@@ -553,17 +553,33 @@ __global__ void half_table_kernel(double* __restrict__ kht, const double2* __res
 }
 
 // out[0] = max |T(d) - T with one axis mirrored|, out[1] = max |T| (bit patterns of
-// non-negative doubles order like integers; a NaN exceeds every number)
-__global__ void even_kernel(const double* __restrict__ T, int W, unsigned long long* __restrict__ out) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= (long long)W * W * W) return;
-  const int a = (int)(i % W), b = (int)((i / W) % W), d = (int)(i / ((long long)W * W));
-  const double t = T[i];
-  const double m[3] = {T[(W - 1 - a) + (long long)W * (b + (long long)W * d)],
-                       T[a + (long long)W * ((W - 1 - b) + (long long)W * d)],
-                       T[a + (long long)W * (b + (long long)W * (W - 1 - d))]};
-  for (int k = 0; k < 3; ++k) atomicMax(out, (unsigned long long)__double_as_longlong(fabs(t - m[k])));
-  atomicMax(out + 1, (unsigned long long)__double_as_longlong(fabs(t)));
+// non-negative doubles order like integers; a NaN exceeds every number).  A CTA's maxima
+// first: with four atomics per value on two words the set-up from a caller's table took 5 ms
+// longer at 63 points a side (15 without) and 10 at 81 (38).
+__global__ void __launch_bounds__(256) even_kernel(const double* __restrict__ T, int W,
+                                                   unsigned long long* __restrict__ out) {
+  __shared__ unsigned long long part[2][8];
+  const long long n = (long long)W * W * W;
+  unsigned long long m[2] = {0, 0};
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const int a = (int)(i % W), b = (int)((i / W) % W), d = (int)(i / ((long long)W * W));
+    const double t = T[i];
+    const double o[3] = {T[(W - 1 - a) + (long long)W * (b + (long long)W * d)],
+                         T[a + (long long)W * ((W - 1 - b) + (long long)W * d)],
+                         T[a + (long long)W * (b + (long long)W * (W - 1 - d))]};
+    for (int k = 0; k < 3; ++k) m[0] = max(m[0], (unsigned long long)__double_as_longlong(fabs(t - o[k])));
+    m[1] = max(m[1], (unsigned long long)__double_as_longlong(fabs(t)));
+  }
+  for (int k = 0; k < 2; ++k) {
+    for (int o = 16; o > 0; o >>= 1) m[k] = max(m[k], __shfl_xor_sync(0xffffffffu, m[k], o));
+    if ((threadIdx.x & 31) == 0) part[k][threadIdx.x >> 5] = m[k];
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    unsigned long long v = 0;
+    for (int w = 0; w < 8; ++w) v = max(v, part[threadIdx.x][w]);
+    atomicMax(out + threadIdx.x, v);
+  }
 }
 
 int make_half(Ctx& c, bool even) {
@@ -583,7 +599,7 @@ int make_half(Ctx& c, bool even) {
     unsigned long long h[2];
     SG_TRY(dalloc(c, &d, sizeof(h)));
     SG_CUDA(cudaMemsetAsync(d, 0, sizeof(h), c.stream));
-    even_kernel<<<ceil_div(W * W * W, 256), 256, 0, c.stream>>>(c.d_tcoul, (int)W, d);
+    even_kernel<<<(int)std::min<long long>(ceil_div(W * W * W, 256), 148 * 8), 256, 0, c.stream>>>(c.d_tcoul, (int)W, d);
     SG_LAUNCHED();
     SG_CUDA(cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, c.stream));
     SG_CUDA(cudaStreamSynchronize(c.stream));
