@@ -252,7 +252,7 @@ template <bool DEN>
 static int launch_rdm(Ctx& c, const long long* off, const int2* ent, const double2* a1, const double2* a2,
                       long long nel, double2* out) {
   const dim3 grid(ceil_div(nel, 4));
-  if (early_evaluation(c.G) && nel <= 20736)
+  if (early_evaluation(c) && nel <= 20736)
     return launch_early(c.stream, rdm_gather_kernel<DEN, true>, grid, dim3(128), 0, off, ent, a1, a2, nel, out);
   rdm_gather_kernel<DEN, false><<<grid, 128, 0, c.stream>>>(off, ent, a1, a2, nel, out);
   SG_LAUNCHED();
@@ -377,7 +377,7 @@ int ci_denmat(Ctx& c, const double2* avec, double2* denmat, double2* invdenmat, 
   SG_CHECK(s.attached, SINCGPU_ESTATE, "no walk tables attached");
   const int n = c.nspf;
   ProfScope ps(c, ST_CI);
-  const bool early = early_evaluation(c.G);
+  const bool early = early_evaluation(c);
   SG_TRY(launch_rdm<true>(c, s.den_off, s.den_ent, avec, avec, (long long)n * n, denmat));
   if (invdenmat) {
     SG_TRY(c.ws_ci2.ensure(sizeof(double2) * n * n + 256));

@@ -84,13 +84,6 @@ template <class... KA, class... A>
 static int launch_early(cudaStream_t stream, void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, A... args) {
   return launch_waiting(stream, true, kernel, grid, block, smem, args...);
 }
-// The two streams of a mean-field evaluation: early up to 41 points a side, where the
-// boundaries count (us per evaluation without and with it: 21^3 / 5 orbitals 65 / 57, 33^3 / 9
-// 321 / 299, 37^3 / 10 493 / 489, 41^3 / 4 165 / 154 waiting for each, 41^3 / 10 569 / 562; with
-// bra and ket apart 33^3 / 9 447 / 429, 41^3 / 4 154 / 141).  Beyond, the waiting CTAs of one
-// stream take room that the other's kernels would use: 44^3 / 12 1042 / 1053, 57^3 / 11 in the
-// mixed form 1429 / 1440, a single 82^3 / 5 1717 / 1791.
-__host__ __device__ constexpr bool early_evaluation(long long points) { return points <= 68921; }
 // acc += v*m with explicit FMAs (one rounding order wherever it is used)
 __device__ __forceinline__ void cfma(double2& acc, double2 v, double2 m) {
   acc.x = fma(v.x, m.x, fma(-v.y, m.y, acc.x));

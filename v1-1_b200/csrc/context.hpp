@@ -199,6 +199,7 @@ struct Ctx {
   CmfState cmf;
   IntCache icache[IC_COUNT];
   cudaGraph_t rhs_graph = nullptr;         // captured orbital-RHS evaluation (graph.cu)
+  bool capturing = false;                  // an evaluation is being captured into it
   cudaGraphExec_t rhs_exec = nullptr;
   int coul_chunk = 0;   // pairs per pass sequence (0 = automatic)
   int coul_fp32 = 0;    // 1: Coulomb passes in FP32 (precision form), 0: FP64
@@ -303,6 +304,17 @@ int make_khat(Ctx& c);
 int ensure_fp32_tables(Ctx& c);
 // real kernel spectrum transposed to [kx][kz][ky] (FP64, and FP32 with fp32)
 int ensure_khT(Ctx& c, bool fp32);
+
+// The two streams of a mean-field evaluation: early up to 41 points a side, where the
+// boundaries count (us per evaluation without and with it: 21^3 / 5 orbitals 65 / 57, 33^3 / 9
+// 321 / 299, 37^3 / 10 493 / 489, 41^3 / 4 165 / 154 waiting for each, 41^3 / 10 569 / 562; with
+// bra and ket apart 33^3 / 9 447 / 429, 41^3 / 4 154 / 141).  Beyond, the waiting CTAs of one
+// stream take room that the other's kernels would use: 44^3 / 12 1042 / 1053, 57^3 / 11 in the
+// mixed form 1429 / 1440, a single 82^3 / 5 1717 / 1791.
+// In a captured graph, whose boundaries are shorter, fewer than 8 orbitals up to 25 (us a
+// replay, ordinary / early: 21^3 / 5 52.5 / 52.5, 31^3 / 5 94 / 102, 37^3 / 4 116 / 134, 41^3 / 6
+// 232 / 247; 25^3 / 8 121.7 / 117.1, 31^3 / 8 184.7 / 181.6, 37^3 / 10 494 / 478, 41^3 / 10 554 / 553).
+inline bool early_evaluation(const Ctx& c) { return c.G <= (c.capturing && c.nspf < 8 ? 15625 : 68921); }
 
 // tables of the half-length Coulomb form for c.d_tcoul; `even`: the kernel is even in
 // each axis by construction (else it is checked)

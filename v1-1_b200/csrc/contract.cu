@@ -801,7 +801,7 @@ int twoe_matel(Ctx& c, const double2* phi1, const double2* phi2, const int* h_pa
     SG_LAUNCHED();
   }
   ProfScope ps(c, ST_TWOE_FINISH);
-  const bool early = early_evaluation(c.G);
+  const bool early = early_evaluation(c);
   SG_TRY(launch_waiting(c.stream, early, split_reduce_kernel, dim3(ceil_div(MM, 32)), dim3(256), 0, part, nsplit, M, TT,
                         C));
   const long long n4 = (long long)n * n * n * n;
@@ -1292,7 +1292,7 @@ static int reduced_pot_impl(Ctx& c, const double* Rpl, const int* h_pa, const in
       const size_t sm = rp_apply_smem(n, NC, fn);
 #define SG_RP_APPLY(FN)                                                                                  \
   case FN:                                                                                               \
-    SG_TRY(launch_waiting(c.stream, early_evaluation(c.G), rp_apply_kernel<FN>, dim3(grid), dim3(256), sm, Rpl, Wm,     \
+    SG_TRY(launch_waiting(c.stream, early_evaluation(c), rp_apply_kernel<FN>, dim3(grid), dim3(256), sm, Rpl, Wm,     \
                           d_rows, packed ? 1 : 0, K, NC, c.G, reducedpot, d_tmap, n, apply->phi, apply->S, apply->inv, \
                           apply->timefac, apply->T));                                                      \
     break;

@@ -512,7 +512,7 @@ int coul_launch(Ctx& c, const CoulArgs<C>& ca, int np, bool dens, const double2*
     }
     return SINCGPU_OK;
   }
-  const bool early = early_evaluation(c.G);
+  const bool early = early_evaluation(c);
   {
     ProfScope ps(c, ST_COUL_FWD_X);
     SG_TRY(launch_waiting(c.stream, early, dens ? coul_fwd_x_t<P1, P2, true, C> : coul_fwd_x_t<P1, P2, false, C>,

@@ -63,7 +63,9 @@ int sincgpu_rhs_graph_capture(sincgpu_ctx* h, const double* phi, const double* a
   int rc = SINCGPU_OK;
   cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
+    c.capturing = true;
     rc = run_rhs(h, a);
+    c.capturing = false;
     cudaGraph_t g = nullptr;
     cudaError_t e2 = cudaStreamEndCapture(cap, &g);
     if (rc == SINCGPU_OK && e2 != cudaSuccess) {
