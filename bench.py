@@ -881,16 +881,15 @@ def secondary_rates(proj, torch, stream, flush, phi, den, inv, red, out, mat, av
 TRAFFIC = {
     ("coul_fwd_x", 41, 10): 70590000, ("coul_fwd_y", 41, 10): 300490000, ("coul_z", 41, 10): 426130000,
     ("coul_inv_y", 41, 10): 323310000, ("coul_inv_x", 41, 10): 143240000, ("twoe_gemm", 41, 10): 72000000,
-    ("rp_gemm", 41, 10): 169050000, ("rhs_redpot", 41, 10): 136340000, ("ke_xy", 41, 10): 12170000,
-    ("ke_z", 41, 10): 22090000,
+    ("rhs_redpot", 41, 10): 136340000, ("ke_xy", 41, 10): 12170000, ("ke_z", 41, 10): 22090000,
 }
 
-# DRAM bytes per pair of a Coulomb z launch on the 81^3 grid (P = 162), from one
-# ncu capture of an 8-pair launch (coul_chunk=8; the full 40-pair launches hold
-# more than the capture size allows): (360.6 + 226.2) MB / 8 pairs.  The W2 slab
-# read and written grows with the pairs (the real spectrum stays in L2), so a
-# launch's traffic is this times its pairs.
-TRAFFIC_PER_PAIR = {("coul_z", 81, 16): 73350000}
+# DRAM bytes per pair of a Coulomb launch on the 81^3 grid (P = 162), each from one ncu
+# capture of an 8-pair launch (coul_chunk=8; the full launches hold more than the capture
+# size allows): z pass (360.6 + 226.2) MB / 8 pairs, plane pass of the half-length form
+# (225.6 + 118.5) MB / 8.  The slab read and written grows with the pairs (the real spectrum
+# stays in L2), so a launch's traffic is this times its pairs.
+TRAFFIC_PER_PAIR = {("coul_z", 81, 16): 73350000, ("coul_yzy", 81, 16): 43010000}
 
 _DGEMM = {}
 
@@ -943,6 +942,13 @@ def coulomb_pass_work(name, N, P, U):
     return by, (lines * fl + extra) * U
 
 
+def contraction_flops(n, G):
+    """Least FP64 flops of twoematel and reducedpot of hermitian pairs: the n^2 real rows of
+    the pair densities (the diagonal pairs have no imaginary part) against the n^2 rows of
+    their potentials, a symmetric product, and against the n^2 real columns of the 2-RDM."""
+    return {"twoe_gemm": float(G) * n * n * (n * n + 1), "rp_gemm": 2.0 * G * n ** 4}
+
+
 def make_roofline(w, prof, nprof, dev, proj_fft_length=None):
     """Dominant kernel of the step (largest summed time in the per-stage profile)
     with its algorithmic bytes or flops per launch.  Coulomb passes and the
@@ -969,7 +975,7 @@ def make_roofline(w, prof, nprof, dev, proj_fft_length=None):
             "traffic": traffic, "traffic_source": src}
     if name in ("rp_gemm", "twoe_gemm", "ke_xy", "ke_z"):
         dgemm = _dgemm_tflops(dev)
-        flops = {"rp_gemm": 2.0 * G * 2 * U * n * (n + 1), "twoe_gemm": 2.0 * G * (2 * U) ** 2,
+        flops = {**contraction_flops(n, G),
                  "ke_xy": 2 * 2 * 2.0 * N ** 3 * N * n, "ke_z": 2 * 2.0 * N ** 3 * N * n}[name] / launches_per_step
         ach = flops / (per_launch_ms / 1e3) / 1e12
         return {**base, "bound": "tensor", "precision": "fp64 (mma.sync f64)", "achieved": ach, "peak": dgemm,
@@ -1013,8 +1019,8 @@ def eval_roofline(w, prof, nprof, dev, P, ms_step):
         # name: (algorithmic bytes, algorithmic flops) per evaluation
         **{k: coulomb_pass_work(k, N, P, U) for k in ("coul_fwd_x", "coul_fwd_y", "coul_z", "coul_inv_y",
                                                       "coul_yzy", "coul_inv_x")},
-        "twoe_gemm": (16.0 * G * (n + 2 * U), 2.0 * G * (2 * U) ** 2),
-        "rp_gemm": (8.0 * G * 2 * U + 16.0 * G * n * n, 2.0 * G * 2 * U * n * (n + 1)),
+        "twoe_gemm": (16.0 * G * n + 8.0 * G * n * n, contraction_flops(n, G)["twoe_gemm"]),
+        "rp_gemm": (8.0 * G * n * n + 16.0 * G * n * n, contraction_flops(n, G)["rp_gemm"]),
         "ke_xy": (16.0 * G * n * 2, 2 * 2 * 2.0 * N ** 3 * N * n),
         "ke_z": (16.0 * G * n * 3, 2 * 2.0 * N ** 3 * N * n),
         "rhs_mix": (16.0 * G * n * 2, 8.0 * G * n * n),
