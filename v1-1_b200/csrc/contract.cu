@@ -1,4 +1,5 @@
-// Dense contractions of the mean-field build, on FP64 CUDA cores.
+// Dense contractions of the mean-field build, on the FP64 tensor cores (register-tiled on the
+// CUDA cores with the options twoe_dmma and rp_dmma off).
 //
 // twoematel (SINCDVR/coreproject.f90:1089-1100):
 //   twoematel(a1,b1,a2,b2) = sum_x rho_{a1b1}(x) R_{a2b2}(x),  rho = phi1_a conj(phi2_b)
@@ -15,7 +16,8 @@
 //       B_p = i(G(c,d)-G(d,c)) for c<d and A_p = G(c,c), B_p = iG(c,c) for c=d,
 //   i.e. [r|s] (G x 2U) times a real 2U x 2n^2 matrix.
 // The n diagonal pairs (c = d) are real, so in FP64 their imaginary rows (zero up to
-// rounding) are left out and 2U = n(n+1) becomes n^2 in both (hermitian_rows).
+// rounding) are left out and 2U = n(n+1) becomes n^2 (hermitian_rows): in reducedpot, and in
+// twoematel where its tiles get smaller.
 // Compared with the complex contractions of the reference this is 4x (twoematel)
 // and 2x (reducedpot) fewer flops.  Without the symmetry (phi1 != phi2) all n^2
 // ordered pairs are used with the plain complex identities.
@@ -973,7 +975,7 @@ __global__ void __launch_bounds__(16 * CG) rp_gemm3_kernel(const double* __restr
 // 16 x 8 FN (2 x FN MMA tiles, 4 FN accumulators per thread), three CTAs per SM,
 // K in chunks of 16 with a two-stage cp.async pipeline (deeper chunks and the
 // third CTA measured faster than 8-deep chunks in three stages at two CTAs per
-// SM).  One column tile covers all n(n+1) columns of the hermitian half for
+// SM).  One column tile covers all columns of the hermitian half (n^2 or n(n+1)) for
 // n <= 10 (FN = 7: 112 columns), so every Rpl row is read once.  Shared-memory rows are padded to 4 (mod 16) doubles so that
 // the fragment loads (lane g + 4t reads row t, column g) are free of bank
 // conflicts.  The accumulator pair (2t, 2t+1) of a fragment is one complex column

@@ -27,10 +27,11 @@
 //   w_L^(n f) = w_2M1^(n1 f) w_2M2^(n2 f) (-1)^(c f)
 // so the y and z transforms of such M are two plain steps, for the odd parity with
 // half-frequency transforms and the sign (-1)^c.  (The x passes keep the first form:
-// its threads read consecutive x.)  The plane kernel is bound by shared-memory
-// wavefronts (81^3: 80 % busy, FP64 pipe 42 %), and the twiddles were a fifth of them;
-// for equal factors of odd M one set per thread serves both directions and parities
-// and stays in registers.
+// its threads read consecutive x.)  The plane kernel's busiest unit is the shared-memory
+// pipe (48^3: 90 % busy, a quarter of it bank conflicts; 81^3: 69 %, FP64 pipe 54 %, with 12
+// warps an SM to cover latency and barriers), and the twiddles were a fifth of its
+// wavefronts; for equal factors of odd M one set per thread serves both directions and
+// parities and stays in registers.
 //
 // Why this form (81^3 grid, 16 orbitals, ms per evaluation): the five passes
 // through HBM (coulomb_kernels.cuh) took 9.7 and were bound by the z pass (4.5), whose
