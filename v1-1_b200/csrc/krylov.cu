@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(kKryThreads) kry_mgs_kernel(double* __restrict
 }
 
 // One Arnoldi step's orthogonalisation on a thread-block cluster: the modified
-// Gram-Schmidt coefficients from one pass of dots (gs_coefficients) instead of
+// Gram-Schmidt coefficients from one pass of dots (gs_solve) instead of
 // kry_mgs_kernel's j + 1 dependent sums.  Row j of L is formed in the same pass over V (v_j
 // is a row already).
 //
@@ -108,8 +108,8 @@ __global__ void __launch_bounds__(kKryThreads) kry_mgs_kernel(double* __restrict
 // two cluster barriers.  The rows' way into shared memory comes before the wait for the
 // sigma product that writes p: that product and the step before may still run (512
 // threads, so that all fit an SM).  After the wait, at 25 rows of 3136 determinants: loads
-// 0.8 us, dots 2.2, barrier 0.7, coefficients 1.5, update 0.9, norm 1.2.  One A-vector step
-// of 30 vectors at 3136 determinants, launches included: 810 -> 527 us, of which clusters of
+// 0.8 us, dots 2.2, barrier 0.7, coefficients 1.3, update 0.9, norm 1.2.  One A-vector step
+// of 30 vectors at 3136 determinants, launches included: 810 -> 522 us, of which clusters of
 // 8 whose rows came from L2 after the sigma product had ended took 14 us a vector.  One CTA
 // with sequential projections is slower at every size: 25 determinants 0.87 ms a step of up
 // to 30 vectors, 0.35 on the cluster; 450 0.95 and 0.38; 3136 1.57 and 0.53.
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(kGsThreads) kry_gs_kernel(double* V, long long
   extern __shared__ __align__(16) double gsm[];  // p, v_j, rows 0 .. cap - 1 of the slice, rows of T
   __shared__ double2 part[kGsCluster][128];  // every CTA's partial dots <v_i, p>, <v_i, v_j>
   __shared__ double2 dots[2][128];           // this CTA's, by halves of its slice
-  __shared__ double npart[kGsCluster], red[kGsThreads / 32], r[128], lrow[128], h[128];
+  __shared__ double npart[kGsCluster], red[kGsThreads / 32], lpart[kGsThreads / 32], r[128], lrow[128], h[128];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rank = cl.block_rank();
   const long long lo = (long long)rank * S;
@@ -230,10 +230,9 @@ __global__ void __launch_bounds__(kGsThreads) kry_gs_kernel(double* V, long long
   }
   __syncthreads();
   // the same in every CTA
-  const double hj = gs_coefficients(
-      j, h, [&](int i) { return r[i]; }, [&](int k) { return lrow[k]; },
-      [&](int i, int k) { return Ts[i * (i - 1) / 2 + k]; }, rank, kGsCluster,
-      [&](int k, double v) { Tm[(long long)j * mh + k] = v; });
+  auto trow = [&](int i, int k) { return Ts[i * (i - 1) / 2 + k]; };
+  auto ldot = [&](int k) { return lrow[k]; };
+  const double hj = gs_solve<kGsThreads / 32>(j, h, lpart, [&](int i) { return r[i]; }, ldot, trow);
   if (rank == 0 && tid <= j) Hm[(long long)j * mh + tid] = tid < j ? h[tid] : hj;
   double s = 0.0;
   const int staged = ALL ? j : cap;
@@ -261,7 +260,9 @@ __global__ void __launch_bounds__(kGsThreads) kry_gs_kernel(double* V, long long
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane < kGsCluster) *cl.map_shared_rank(&npart[rank], lane) = s;
   }
-  cl.sync();
+  auto arrived = cl.barrier_arrive();
+  gs_extend(j, ldot, trow, rank, kGsCluster, [&](int k, double v) { Tm[(long long)j * mh + k] = v; });
+  cl.barrier_wait(std::move(arrived));
   double t = 0.0;
 #pragma unroll
   for (int q = 0; q < kGsCluster; ++q) t += npart[q];

@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(kLvThreads, 2) lv_arnoldi_orth_kernel(const do
 // The orthogonalisation of Arnoldi step j in three launches of any length (option
 // orth_onepass): the coefficients of the modified Gram-Schmidt from one pass of dots.
 // With r_i = <v_i, p> and row j of L, <v_j, v_k>, summed in one pass (v_j is a row already),
-// gs_coefficients forms them.
+// gs_solve forms them.
 //   lv_dots_all: r and row j of L, eight rows of V at a time in registers; the last CTA
 //                adds the partials in a fixed order and forms h
 //   lv_project:  p -= sum_i h_i v_i and |p|^2; the last CTA sets h(j+1,j) and breakdown
@@ -296,14 +296,15 @@ __device__ __forceinline__ bool lv_last_cta(unsigned* count, unsigned* sh) {
 
 // totals of the 2 (j + 1) dots over the CTAs' partials in a fixed order, the coefficients h
 // and elements k0, k0 + kstep, ... of row j of T; one CTA
-__device__ __forceinline__ void lv_coefficients(const double* part, int j, double* tot, double* h, double* Tm, int mh,
+__device__ __forceinline__ void lv_coefficients(const double* sums, int j, double* tot, double* h, double* Tm, int mh,
                                                 int k0, int kstep) {
+  __shared__ double part[kLvThreads / 32];
   constexpr int U = (kLvBlocks + 31) / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int e = warp; e < 2 * (j + 1); e += kLvThreads / 32) {
     double v[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) v[u] = lane + 32 * u < kLvBlocks ? __ldcg(part + (long long)e * kLvBlocks + lane + 32 * u) : 0.0;
+    for (int u = 0; u < U; ++u) v[u] = lane + 32 * u < kLvBlocks ? __ldcg(sums + (long long)e * kLvBlocks + lane + 32 * u) : 0.0;
     double s = 0.0;
 #pragma unroll
     for (int u = 0; u < U; ++u) s += v[u];
@@ -311,10 +312,10 @@ __device__ __forceinline__ void lv_coefficients(const double* part, int j, doubl
     if (lane == 0) tot[e] = s;
   }
   __syncthreads();
-  const double hj = gs_coefficients(
-      j, h, [&](int i) { return tot[2 * i]; }, [&](int k) { return tot[2 * k + 1]; },
-      [&](int i, int k) { return Tm[(long long)i * mh + k]; }, k0, kstep,
-      [&](int k, double v) { Tm[(long long)j * mh + k] = v; });
+  auto trow = [&](int i, int k) { return Tm[(long long)i * mh + k]; };
+  auto ldot = [&](int k) { return tot[2 * k + 1]; };
+  const double hj = gs_solve<kLvThreads / 32>(j, h, part, [&](int i) { return tot[2 * i]; }, ldot, trow);
+  gs_extend(j, ldot, trow, k0, kstep, [&](int k, double v) { Tm[(long long)j * mh + k] = v; });
   if (threadIdx.x == 0) h[j] = hj;
   __syncthreads();
 }
@@ -660,7 +661,7 @@ struct OrbWork {
   double2 *V, *jv, *jvo, *u, *w, *T, *tmp, *dpart;
   double2 *D2, *M1, *ovl, *smh;
   double *part0, *part1, *Hm, *exph, *Efull, *pscratch, *err;
-  double *gpart, *Tm;  // lv_dots_all_kernel's partials, gs_coefficients' T
+  double *gpart, *Tm;  // lv_dots_all_kernel's partials, gs_solve's T
   OrbKryState* st;
   int* ns;
   unsigned* gbar;  // lv_arnoldi_orth_kernel's grid barrier (count, generation), lv_last_cta's count
